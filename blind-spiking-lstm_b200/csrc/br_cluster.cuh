@@ -93,8 +93,7 @@ __global__ void __launch_bounds__(BR_CLUSTER_THREADS, 1) br_cluster_kernel(const
     double2* outp = spec + LH * H;                           // [H]
     double2* qt_s = outp + H;                                // N / 2, swizzled
     double2* tw = qt_s + N / 2;                              // PL::TW
-    uint16_t* freq = reinterpret_cast<uint16_t*>(tw + PL::TW);
-    int* rot_all = reinterpret_cast<int*>(freq + H);         // G * M
+    int* rot_all = reinterpret_cast<int*>(tw + PL::TW);      // G * M
     int* bexp = rot_all + (size_t)args.G * M;                // 1
     auto qtab = [&](int x) { return qt_s[qsw<LOGN>(x)]; };
 
@@ -110,7 +109,6 @@ __global__ void __launch_bounds__(BR_CLUSTER_THREADS, 1) br_cluster_kernel(const
 
     for (int i = tid; i < N / 2; i += nt) qt_s[qsw<LOGN>(i)] = args.qt[i];
     for (int i = tid; i < PL::TW; i += nt) tw[i] = args.tw[i];
-    for (int i = tid; i < H; i += nt) freq[i] = args.freq[i];
     uint32_t spec_of[2 * S];                                 // digit spectra of each rank
 #pragma unroll
     for (int k = 0; k < 2 * S; ++k) spec_of[k] = peer_smem(spec, (uint32_t)k);
@@ -118,6 +116,12 @@ __global__ void __launch_bounds__(BR_CLUSTER_THREADS, 1) br_cluster_kernel(const
 #pragma unroll
     for (int k = 0; k < S; ++k) out_of[k] = peer_smem(outp, (uint32_t)(r + 2 * k));
     cluster_barrier();                                       // every CTA of the cluster has started
+
+    // this thread's key slot in the pointwise stage (a part's slots are its
+    // positions): where its digits lie, and its evaluation point zeta^e
+    const int u0 = h * PART + tid / TPS;
+    const int pat = swz(key_pos<LOGH>(u0));
+    const int e = 4 * args.freq[key_pos<LOGH>(u0)] + 1;
 
     const bool owner = tid < Q8;
     const int on1 = tid;
@@ -265,20 +269,17 @@ __global__ void __launch_bounds__(BR_CLUSTER_THREADS, 1) br_cluster_kernel(const
             // out = sum_m X^{r_m} * sum_bc BSK[g, r, bc, m] * DEC[bc]
             {
                 const size_t gbase = (size_t)g * 2 * P * M * H;
-                const int p = h * PART + tid / TPS;
                 double2 d[P];
 #pragma unroll
                 for (int lvl = 0; lvl < L; ++lvl)
 #pragma unroll
                     for (int in = 0; in < 2; ++in) {
                         const int src = in + 2 * (lvl % S);          // rank holding digit (lvl, in)
-                        const int e_off = (lvl / S) * H + swz(p);
+                        const int e_off = (lvl / S) * H + pat;
                         d[2 * lvl + in] = src == rank ? spec[e_off]
                                                       : ld_peer(spec_of[src] + (uint32_t)(e_off * sizeof(double2)));
                     }
-                const int j = freq[p];
-                const int e = 4 * j + 1;
-                const double2* kb2 = args.bsk + gbase + 2 * (size_t)p + (size_t)r * (P / 2) * M * H * 2;
+                const double2* kb2 = args.bsk + gbase + 2 * (size_t)u0 + (size_t)r * (P / 2) * M * H * 2;
                 double2 o = make_double2(0.0, 0.0);
                 if constexpr (TPS == 1) {
                     // br_split_kernel's contraction: the key words of MC
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(BR_CLUSTER_THREADS, 1) br_cluster_kernel(const
                                 c_mac(o, w, t);
                             }
                     }
-                    outp[swz(p)] = o;
+                    outp[pat] = o;
                 } else {
                     // lane u of the position contracts patterns
                     // [u M/TPS, (u+1) M/TPS) (M a multiple of TPS); lane 0
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(BR_CLUSTER_THREADS, 1) br_cluster_kernel(const
                                 }
                         }
                     }
-                    if (u == TPS - 1) outp[swz(p)] = o;
+                    if (u == TPS - 1) outp[pat] = o;
                 }
             }
             __syncthreads();

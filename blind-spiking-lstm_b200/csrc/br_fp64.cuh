@@ -463,7 +463,8 @@ __global__ void __launch_bounds__(KR > 0 ? KR * (1 << LOGN) / 8 : 512, 1) br_fp6
                 const int KG = K / KT;
                 for (int t = tid; t < KG * H; t += nt) {
                     const int kg = t % KG;
-                    const int p = t / KG;
+                    const int u = t / KG;                          // key slot (the reference layout has position order)
+                    const int p = REFLAYOUT ? u : key_pos<LOGH>(u);
                     double2 d[KT][P];
     #pragma unroll
                     for (int kt = 0; kt < KT; ++kt)
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(KR > 0 ? KR * (1 << LOGN) / 8 : 512, 1) br_fp6
     #pragma unroll
                     for (int kt = 0; kt < KT; ++kt) o0[kt] = o1[kt] = make_double2(0.0, 0.0);
                     const double2* kb = args.bsk + gbase + jr;          // reference layout
-                    const double2* kb2 = args.bsk + gbase + 2 * (size_t)p; // native: pairs of digits
+                    const double2* kb2 = args.bsk + gbase + 2 * (size_t)u; // native: pairs of digits
 #pragma unroll 1
                     for (int m = 0; m < M; ++m) {
                         if (args.prefetch > 0 || (args.prefetch < 0 && 2 * P * KT > 16)) {
@@ -727,8 +728,8 @@ __global__ void __launch_bounds__(KR > 0 ? KR * (1 << LOGN) / 8 : 512, 1) br_fp6
 
 // ----------------------------------------------------------------------------
 // Forward FFT of the coefficient-domain bootstrapping key into the device
-// layout [G][2 out][P/2][M][H][2] (position order; the two digits bc = 2j,
-// 2j+1 of a slot adjacent), P = 2L, bc = level * 2 + in.
+// layout [G][2 out][P/2][M][H][2] (slot order, key_pos; the two digits bc =
+// 2j, 2j+1 of a slot adjacent), P = 2L, bc = level * 2 + in.
 // Source: uint32 (2 in = left/right, 2 out = mask/body, G*M, L, N), the
 // layout of get_boostrapping_key_collapse (schemas/RLWE_jax.py:162-197).
 // The reference transforms the same integers with jax_fourier and permutes
@@ -793,7 +794,7 @@ __global__ void __launch_bounds__(256) bsk_fft_kernel(const BskConvArgs a) {
             di = ((((size_t)g * parts + p / a.ring_nt) * 2 + out) * a.M + m) * P + bc;
             di = di * a.ring_nt + p % a.ring_nt;
         } else {
-            di = ((((size_t)(g * 2 + out) * (P / 2) + bc / 2) * a.M + m) * H + p) * 2 + (bc & 1);
+            di = ((((size_t)(g * 2 + out) * (P / 2) + bc / 2) * a.M + m) * H + key_slot<LOGH>(p)) * 2 + (bc & 1);
         }
         // times 1/H: a power of two, so every product and sum of the blind
         // rotation comes out exactly 1/H times the unscaled one, and the

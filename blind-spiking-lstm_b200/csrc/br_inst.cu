@@ -3,6 +3,7 @@
 #include "br_cluster.cuh"
 #include "br_split.cuh"
 #include "br_tm.cuh"
+#include "br_warp.cuh"
 #include "tfhe_dispatch.h"
 
 #ifndef BR_LOGN
@@ -97,6 +98,8 @@ BrKernel br_tm32_logn11(int L) {
         default: return nullptr;
     }
 }
+
+BrKernel br_warp32_logn11(int NP) { return NP == 2 ? br_warp_kernel<false, 2> : br_warp_kernel<false, 1>; }
 #endif
 
 }  // namespace tfhe

@@ -6,6 +6,7 @@
 #include "br_cluster.cuh"
 #include "br_split.cuh"
 #include "br_tm.cuh"
+#include "br_warp.cuh"
 #include "tfhe_dispatch.h"
 
 #ifndef BR_LOGN
@@ -76,6 +77,8 @@ BrKernel br_tm64_logn11(int L) {
         default: return nullptr;
     }
 }
+
+BrKernel br_warp64_logn11() { return br_warp_kernel<true, 2>; }
 #endif
 
 }  // namespace tfhe

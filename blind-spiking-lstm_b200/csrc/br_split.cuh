@@ -108,8 +108,7 @@ __global__ void __launch_bounds__(BR_SPLIT_THREADS, 1) br_split_kernel(const BrA
     double2* outp = spec + 2 * L * H;                        // [H]
     double2* qt_s = outp + H;                                // N / 2, swizzled
     double2* tw = qt_s + N / 2;                              // PL::TW
-    uint16_t* freq = reinterpret_cast<uint16_t*>(tw + PL::TW);
-    int* rot_all = reinterpret_cast<int*>(freq + H);         // G * M
+    int* rot_all = reinterpret_cast<int*>(tw + PL::TW);      // G * M
     int* bexp = rot_all + (size_t)args.G * M;                // 1
     auto qtab = [&](int r) { return qt_s[qsw<LOGN>(r)]; };
 
@@ -122,9 +121,19 @@ __global__ void __launch_bounds__(BR_SPLIT_THREADS, 1) br_split_kernel(const BrA
 
     for (int i = tid; i < N / 2; i += nt) qt_s[qsw<LOGN>(i)] = args.qt[i];
     for (int i = tid; i < PL::TW; i += nt) tw[i] = args.tw[i];
-    for (int i = tid; i < H; i += nt) freq[i] = args.freq[i];
     const uint32_t peer_spec = peer_smem(spec, (uint32_t)(r ^ 1));
     cluster_barrier();                                       // the peer has started
+
+    // this thread's key slots in the pointwise stage: where their digits lie,
+    // and their evaluation points zeta^e
+    constexpr int SL = H > BR_SPLIT_THREADS ? H / BR_SPLIT_THREADS : 1;
+    int at[SL], ev[SL];
+#pragma unroll
+    for (int sl = 0; sl < SL; ++sl) {
+        const int p = key_pos<LOGH>((tid + sl * BR_SPLIT_THREADS) % H);
+        at[sl] = swz(p);
+        ev[sl] = 4 * args.freq[p] + 1;
+    }
 
     const bool owner = tid < Q8;
     const int on1 = tid;
@@ -266,20 +275,22 @@ __global__ void __launch_bounds__(BR_SPLIT_THREADS, 1) br_split_kernel(const BrA
             // pointwise: output r = sum_m X^{r_m} * sum_bc BSK[g, r, bc, m] * DEC[bc]
             {
                 const size_t gbase = (size_t)g * 2 * P * M * H;
-                for (int p = tid; p < H; p += nt) {
+#pragma unroll
+                for (int sl = 0; sl < SL; ++sl) {
+                    const int u = tid + sl * BR_SPLIT_THREADS;
+                    if (SL == 1 && u >= H) break;
                     double2 d[P];
 #pragma unroll
                     for (int lvl = 0; lvl < L; ++lvl) {
-                        const double2 own = mine_spec[lvl * H + swz(p)];
+                        const double2 own = mine_spec[lvl * H + at[sl]];
                         const double2 other =
-                            ld_peer(peer_base + (uint32_t)((lvl * H + swz(p)) * sizeof(double2)));
+                            ld_peer(peer_base + (uint32_t)((lvl * H + at[sl]) * sizeof(double2)));
                         d[2 * lvl + r] = own;
                         d[2 * lvl + (r ^ 1)] = other;
                     }
-                    const int j = freq[p];
-                    const int e = 4 * j + 1;
+                    const int e = ev[sl];
                     double2 o = make_double2(0.0, 0.0);
-                    const double2* kb2 = args.bsk + gbase + 2 * (size_t)p + (size_t)r * (P / 2) * M * H * 2;
+                    const double2* kb2 = args.bsk + gbase + 2 * (size_t)u + (size_t)r * (P / 2) * M * H * 2;
                     // one ciphertext per SM leaves little to hide a key load's
                     // latency behind: the key words of MC patterns are all in
                     // flight before the first of them is contracted (the
@@ -307,7 +318,7 @@ __global__ void __launch_bounds__(BR_SPLIT_THREADS, 1) br_split_kernel(const BrA
                                 c_mac(o, w, t);
                             }
                     }
-                    outp[swz(p)] = o;
+                    outp[at[sl]] = o;
                 }
             }
             __syncthreads();

@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(BR_TM_THREADS, 1) br_tm_kernel(const BrArgs ar
             // word loaded serves K of them
             {
                 const size_t gbase = (size_t)g * 2 * P * M * H;
-                for (int p = tid; p < H; p += nt) {
+                for (int u = tid; u < H; u += nt) {
+                    const int p = key_pos<LOGH>(u);
                     double2 d[K][P];
 #pragma unroll
                     for (int kt = 0; kt < K; ++kt)
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(BR_TM_THREADS, 1) br_tm_kernel(const BrArgs ar
                     double2 o0[K], o1[K];
 #pragma unroll
                     for (int kt = 0; kt < K; ++kt) o0[kt] = o1[kt] = make_double2(0.0, 0.0);
-                    const double2* kb2 = args.bsk + gbase + 2 * (size_t)p;
+                    const double2* kb2 = args.bsk + gbase + 2 * (size_t)u;
 #pragma unroll 1
                     for (int m = 0; m < M; ++m) {
                         // both outputs' key words of this pattern in flight, then

@@ -582,6 +582,55 @@ static int launch_tm(const BrArgs& args, int N, int L, cudaStream_t stream, cons
     return check_cuda(cudaGetLastError(), "blind rotation launch (tensor memory)");
 }
 
+// The warp-local kernel (br_warp.cuh) takes N = 2048, l_bs = 2 in the native
+// layout, NP pairs of ciphertexts per CTA.
+static bool warp_form(int N, int L, int G, int M, int NP, bool reflayout, int kr) {
+    return !reflayout && kr == 0 && N == 2048 && L == 2 && M >= 2 && M % 2 == 0 &&
+           br_warp_smem(NP, G, M) <= (size_t)max_smem_optin();
+}
+
+// TFHE_B200_PERSISTENT=0 (or the keys' tuning) launches one CTA per set
+static bool persistent_launch(const tfhe_tuning* tune) {
+    static const bool env_on = [] {
+        const char* env = getenv("TFHE_B200_PERSISTENT");
+        return !(env && env[0] == '0');
+    }();
+    return (tune && tune->persistent >= 0) ? tune->persistent != 0 : env_on;
+}
+
+// Ciphertexts of a batch that go to the four-per-CTA kernel in automatic
+// shapes: whole rounds of 4 per SM, and the rest too where a partly filled
+// round is the shortest way (n=742 N=2048, cycles per group and round: four
+// per CTA 44.3k, two 23.4k, one 20.6k; with eight patterns 60.8k, 36.5k and
+// about 30k): above three per SM, with more than four patterns above two.
+static long long warp_four_share(int N, int L, int G, int M, long long B, bool reflayout, int kr,
+                                 const tfhe_tuning* tune) {
+    const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
+    if (requested || !persistent_launch(tune) || !warp_form(N, L, G, M, 2, reflayout, kr)) return 0;
+    const long long sms = std::max(1, sm_count());
+    const long long full = B / (4 * sms) * (4 * sms);
+    return B - full > (M <= 4 ? 3 : 2) * sms ? B : full;
+}
+
+static int launch_warp_four(const BrArgs& args, int N, cudaStream_t stream, const tfhe_tuning* tune) {
+    BrKernel kern = br_warp_kernel_for(args.lwe_a64 != nullptr, 2);
+    const size_t smem = br_warp_smem(2, args.G, args.M);
+    int per_sm = 1;
+    TFHE_TRY(prepare_kernel((const void*)kern, BW_THREADS, smem, &per_sm));
+    BrArgs a = args;
+    const FftPlan* pl = get_plan(N);
+    if (!pl) return TFHE_ERR_INTERNAL;
+    a.qt = pl->qt;
+    a.tw = pl->tw;
+    a.freq = pl->freq;
+    a.K = 4;
+    a.l2_prefetch = (tune && tune->l2_prefetch == 0) ? 0 : 1;
+    const long long sets = (args.B + 3) / 4;
+    count_launch();
+    kern<<<(unsigned)std::min<long long>(sets, std::max(1, sm_count())), BW_THREADS, smem, stream>>>(a);
+    return check_cuda(cudaGetLastError(), "blind rotation launch (four per CTA)");
+}
+
 static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStream_t stream,
                      int* status = nullptr, const tfhe_tuning* tune = nullptr) {
     const int logn = ilog2(N);
@@ -603,12 +652,31 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
             return launch_br(args_after(args, full, N), N, L, reflayout, kr, stream, status, &rest_tune);
         }
     }
+    if (const long long four = warp_four_share(N, L, args.G, args.M, args.B, reflayout, kr, tune)) {
+        BrArgs head = args;
+        head.B = four;
+        TFHE_TRY(launch_warp_four(head, N, stream, tune));
+        if (four == args.B) return TFHE_OK;
+        return launch_br(args_after(args, four, N), N, L, reflayout, kr, stream, status, tune);
+    }
     const BrShape sh = kr > 0 ? ring_shape(N, L, args.M)
                               : br_shape(N, L, args.M, args.B, tune ? tune->ciphertexts_per_cta : 0, !reflayout);
     if (kr > 0 && sh.kr != kr) return fail(TFHE_ERR_INVALID_ARGUMENT, "key ring layout not available for these keys");
     const bool t64 = args.lwe_a64 != nullptr;
-    BrKernel kern = t64 ? (kr == 0 ? br_fp64_t64_kernel_for(logn, L, sh.kt, sh.qtg, sh.xt) : nullptr)
-                        : br_fp64_kernel_for(logn, L, reflayout, kr, sh.kt, sh.qtg, sh.xt);
+    BrKernel kern = nullptr;
+    int nt = sh.nt;
+    size_t smem = sh.smem;
+    // two ciphertexts per CTA on the 32-bit torus: the warp-local kernel's
+    // one-pair form (n=742: 23.4k against 25.9k cycles per group; with the
+    // eight patterns of the 64-bit torus it gains nothing, 36.9k against 36.5k)
+    if (!t64 && sh.K == 2 && !sh.xt && !sh.qtg && warp_form(N, L, args.G, args.M, 1, reflayout, kr)) {
+        kern = br_warp_kernel_for(false, 1);
+        nt = BW_THREADS;
+        smem = br_warp_smem(1, args.G, args.M);
+    } else {
+        kern = t64 ? (kr == 0 ? br_fp64_t64_kernel_for(logn, L, sh.kt, sh.qtg, sh.xt) : nullptr)
+                   : br_fp64_kernel_for(logn, L, reflayout, kr, sh.kt, sh.qtg, sh.xt);
+    }
     if (!kern) return fail(TFHE_ERR_INVALID_ARGUMENT, "unsupported degree / levels");
     if (sh.K < 1)
         return fail(TFHE_ERR_INVALID_ARGUMENT,
@@ -636,16 +704,12 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
     args.status = status ? status : device_status_word();
     if (!args.status) return fail(TFHE_ERR_INTERNAL, "device status word unavailable");
     int per_sm = 1;
-    TFHE_TRY(prepare_kernel((const void*)kern, sh.nt, sh.smem, &per_sm));
+    TFHE_TRY(prepare_kernel((const void*)kern, nt, smem, &per_sm));
     // persistent CTAs: as many as fit on the SMs, looping over ciphertext
     // sets, so all SMs walk the key in lockstep; TFHE_B200_PERSISTENT=0 (or
     // the keys' tuning) launches one CTA per set instead
     const long long sets = (args.B + sh.K - 1) / sh.K;
-    static const bool persistent_env = [] {
-        const char* env = getenv("TFHE_B200_PERSISTENT");
-        return !(env && env[0] == '0');
-    }();
-    const bool persistent = (tune && tune->persistent >= 0) ? tune->persistent != 0 : persistent_env;
+    const bool persistent = persistent_launch(tune);
     const long long grid = persistent ? std::min<long long>(sets, (long long)sm_count() * per_sm) : sets;
     // A last round of at most one ciphertext per SM runs as its own launch of
     // the small-batch shape (one ciphertext per CTA, 512 threads): that is
@@ -658,13 +722,13 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
             BrArgs head = args;
             head.B = full;
             count_launch();
-            kern<<<(unsigned)grid, sh.nt, sh.smem, stream>>>(head);
+            kern<<<(unsigned)grid, nt, smem, stream>>>(head);
             TFHE_TRY(check_cuda(cudaGetLastError(), "blind rotation launch"));
             return launch_br(args_after(args, full, N), N, L, reflayout, 0, stream, status, tune);
         }
     }
     count_launch();
-    kern<<<(unsigned)grid, sh.nt, sh.smem, stream>>>(args);
+    kern<<<(unsigned)grid, nt, smem, stream>>>(args);
     return check_cuda(cudaGetLastError(), "blind rotation launch");
 }
 
@@ -1109,7 +1173,7 @@ int tfhe_keys_create_fourier(const tfhe_params* params, const double* bsk_ordere
     std::vector<uint16_t> freq;
     build_tables(N, qt, tw, freq);
     // bsk_ordered (2 out, 2 in, L, G*M, H) at zeta^(2j+1) -> [G][2][P/2][M][H][2]
-    // at zeta^(4 freq[p] + 1) (the point or the conjugate of its partner)
+    // (slot order, key_pos) at zeta^(4 freq[p] + 1) (the point or the conjugate of its partner)
     const size_t total = (size_t)G * 2 * P * M * H;
     std::vector<double2> host(total);
     const double2* src = reinterpret_cast<const double2*>(bsk_ordered);
@@ -1129,7 +1193,8 @@ int tfhe_keys_create_fourier(const tfhe_params* params, const double* bsk_ordere
                                 di = ((((size_t)g * (H / rnt) + pp / rnt) * 2 + a) * M + m) * P + bc;
                                 di = di * rnt + pp % rnt;
                             } else {
-                                di = (((((size_t)g * 2 + a) * (P / 2) + bc / 2) * M + m) * H + pp) * 2 + (bc & 1);
+                                const int u = H == 1024 ? key_slot<10>(pp) : pp;
+                                di = (((((size_t)g * 2 + a) * (P / 2) + bc / 2) * M + m) * H + u) * 2 + (bc & 1);
                             }
                             // times 1/H, as bsk_fft_kernel stores the native key
                             const double2 w = e < N ? row[2 * j] : make_double2(row[N - 1 - 2 * j].x, -row[N - 1 - 2 * j].y);
@@ -1332,7 +1397,9 @@ int tfhe_pbs_host(const tfhe_keys* keys, const uint32_t* a_host, const uint32_t*
     if (C == 0) {
         const BrShape sh = br_shape(p.N, p.l_bs, keys->M, std::max<long long>(batch, 1 << 20),
                                     keys->tune.ciphertexts_per_cta, true);
-        const long long wave = (long long)std::max(1, sm_count()) * std::max(1, sh.K) * (sh.qtg ? 2 : 1);
+        const long long per_sm = warp_four_share(p.N, p.l_bs, keys->G, keys->M, 1 << 20, false, keys->ring_kr, &keys->tune)
+                                     ? 4 : std::max(1, sh.K) * (sh.qtg ? 2 : 1);
+        const long long wave = (long long)std::max(1, sm_count()) * per_sm;
         C = std::max<long long>(wave, ((batch + 7) / 8 + wave - 1) / wave * wave);
     }
     C = std::min<long long>(C, batch);

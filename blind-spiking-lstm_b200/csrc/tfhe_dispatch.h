@@ -5,6 +5,7 @@
 #include "br_cluster.cuh"
 #include "br_split.cuh"
 #include "br_tm.cuh"
+#include "br_warp.cuh"
 
 namespace tfhe {
 
@@ -84,6 +85,12 @@ inline BrKernel br_tm_kernel_for(int logn, int L, bool t64) {
     if (logn != 11) return nullptr;
     return t64 ? br_tm64_logn11(L) : br_tm32_logn11(L);
 }
+
+// the warp-local kernels (NP pairs of ciphertexts per CTA), N = 2048, l_bs = 2;
+// one pair on the 32-bit torus only
+BrKernel br_warp32_logn11(int NP);
+BrKernel br_warp64_logn11();
+inline BrKernel br_warp_kernel_for(bool t64, int NP) { return t64 ? br_warp64_logn11() : br_warp32_logn11(NP); }
 
 inline BrConvKernel bsk_fft_kernel_for(int logn) {
     switch (logn) {

@@ -104,13 +104,40 @@ struct Plan {
 // stage take the minimum of 4 wavefronts per 32 16-byte requests.
 __device__ __forceinline__ int swz(int e) { return e ^ (((e >> 3) ^ (e >> 4)) & 7); }
 
+// Storage order of the native Fourier key's H slots: slot u holds position
+// key_pos(u).  At H = 1024 it is the order in which br_warp_kernel's warps
+// contract: slot (warp w, step s, lane) = w 128 + s 32 + lane, so one warp's
+// loads of a step are 1 KB in a row; w, s and lane name the digits of the
+// position (superstages 8.8.16) as that kernel holds them.  The other degrees
+// keep position order.
+template <int LOGH>
+__host__ __device__ __forceinline__ int key_pos(int u) {
+    if constexpr (LOGH != 10) return u;
+    const int w = u >> 7, s = (u >> 5) & 3, g = u & 15;
+    const int k0 = ((w >> 1) << 1) | ((u >> 4) & 1);                             // first superstage's digit
+    const int k1 = (w & 1) | (((g >> 3) & 1) << 1) | (((g >> 2) & 1) << 2);      // second's
+    const int k2 = ((s & 1) << 3) | ((s >> 1) << 2) | ((g & 1) << 1) | ((g >> 1) & 1);   // third's
+    return k0 * 128 + k1 * 16 + k2;
+}
+// its inverse
+template <int LOGH>
+__host__ __device__ __forceinline__ int key_slot(int p) {
+    if constexpr (LOGH != 10) return p;
+    const int k0 = p >> 7, k1 = (p >> 4) & 7, k2 = p & 15;
+    const int w = ((k0 >> 1) << 1) | (k1 & 1);
+    const int s = ((k2 >> 3) & 1) | (((k2 >> 2) & 1) << 1);
+    const int g = (((k1 >> 1) & 1) << 3) | (((k1 >> 2) & 1) << 2) | ((k2 & 1) << 1) | ((k2 >> 1) & 1);
+    return w * 128 + s * 32 + (k0 & 1) * 16 + g;
+}
+
 // slot of root r in the swizzled shared-memory quarter table: the low three
-// bits (16-byte bank group) are XORed with bits 3.. and bits log2 N - 3..,
+// bits (16-byte bank group) are XORed with bits 3.. and bits log2 N - 4..,
 // so both a warp's run of consecutive roots and the X^r lookups of one
-// pointwise pass (roots N/8 apart) fall in distinct bank groups
+// pointwise pass (roots N/8 apart, N/16 in the slot order of N = 2048) fall in
+// distinct bank groups
 template <int LOGN>
 __device__ __forceinline__ int qsw(int r) {
-    return r ^ (((r >> 3) ^ (r >> (LOGN - 3))) & 7);
+    return r ^ (((r >> 3) ^ (r >> (LOGN - 4))) & 7);
 }
 
 // exp(-i pi idx / N) for any idx, from the quarter table qt[r] =

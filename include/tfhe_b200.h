@@ -116,8 +116,10 @@ int tfhe_keys_create_fourier(const tfhe_params* params, const double* bsk_ordere
 void tfhe_keys_destroy(tfhe_keys* keys);
 
 /* Set (NULL: reset to automatic) the launch shape used by this key set's
- * blind rotations, and query the shape a batch would get.  Tuning only
- * changes speed, never results (no counterpart in the reference). */
+ * blind rotations, and query the shape a batch would get from the general
+ * one-CTA kernel (the cluster forms of small batches and the warp-local form
+ * of large ones at N = 2048 have shapes of their own).  Tuning only changes
+ * speed, never results (no counterpart in the reference). */
 int tfhe_keys_set_tuning(tfhe_keys* keys, const tfhe_tuning* tuning);
 int tfhe_keys_launch_shape(const tfhe_keys* keys, int64_t batch, int32_t* ciphertexts_per_cta,
                            int32_t* threads, int64_t* shared_bytes);

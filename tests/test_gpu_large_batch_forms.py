@@ -1,0 +1,58 @@
+"""The large-batch forms of the blind rotation (several ciphertexts per CTA
+sharing each key word) against the one-ciphertext-per-CTA form, bit for bit:
+the same operations on every value, so no tolerance."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from tfhe_b200 import client, client64                      # noqa: E402
+from tfhe_b200.engine import Keys                           # noqa: E402
+from tfhe_b200.params import ParamSet                       # noqa: E402
+
+
+def _batches():
+    """One round of four per SM less and more one, the remainders on either
+    side of each choice of form, and several rounds."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return [sms + 1, 2 * sms, 2 * sms + 1, 3 * sms, 3 * sms + 1, 4 * sms - 1, 4 * sms, 4 * sms + 1, 9 * sms + 3]
+
+
+def _compare(keys, p, word, n, batch, n_lut, seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    info = torch.iinfo(word)
+    draw = lambda shape: torch.randint(info.min, info.max, shape, device="cuda", generator=g, dtype=word)
+    a, b = draw((batch, n)), draw((batch,))
+    for count in (1, batch):
+        lut = draw((count, 2, p.N))
+        keys.set_tuning()
+        got = keys.cuboot_merge(a, b, lut, n_lut)
+        acc = keys.blind_rotate(a, b, lut, n_lut)
+        keys.set_tuning(ciphertexts_per_cta=1)
+        want = keys.cuboot_merge(a, b, lut, n_lut)
+        acc1 = keys.blind_rotate(a, b, lut, n_lut)
+        keys.set_tuning()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), (batch, n_lut, count)
+        assert torch.equal(acc, acc1), (batch, n_lut, count)
+
+
+@pytest.mark.parametrize("collapse", [1, 2, 3, 4])
+def test_n2048_l2_matches_one_per_cta(collapse):
+    p = ParamSet("n12_N2048", N=2048, n=12, log2_beta_bs=15, l_bs=2, collapse=collapse, log2_beta_ks=4, l_ks=5,
+                 sigma_glwe=1.0, sigma_lwe=2.0 ** 15)
+    k = client.keygen(p, collapse)
+    keys = Keys.create(p, k.bsk, k.ksk_a, k.ksk_b)
+    for i, batch in enumerate(_batches()):
+        _compare(keys, p, torch.int32, p.n, batch, (1, 4)[i % 2], 100 * collapse + i)
+
+
+@pytest.mark.parametrize("collapse", [1, 3])
+def test_n2048_l2_torus64_matches_one_per_cta(collapse):
+    from tfhe_b200.torus64 import Keys64
+    p = client64.Params64("n12_N2048_q64", N=2048, n=12, log2_beta_bs=13, l_bs=2, collapse=collapse, log2_beta_ks=4,
+                          l_ks=5, sigma_glwe=2.0 ** 17, sigma_lwe=2.0 ** 40)
+    keys = Keys64(client64.keygen(p, collapse))
+    for i, batch in enumerate(_batches()):
+        _compare(keys, p, torch.int64, p.n, batch, (1, 4)[i % 2], 100 * collapse + i)
