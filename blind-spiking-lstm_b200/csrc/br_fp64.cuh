@@ -32,6 +32,7 @@ constexpr bool br_extra_threads(int L) { return L <= 3; }
 
 struct BrArgs {
     const double2* bsk;       // native [G][2][P/2][M][H][2]; reference layout (G,2,L,2,M,H)
+    const double* bsk_mma;    // the same key in br_mma_kernel's layout (nullptr: none)
     const double2* all_rot;   // reference layout only: (2N, H)
     const double2* qt;
     const double2* qr;        // qt in rotation order (rot_slot): the QTG layout's only root table

@@ -1,6 +1,7 @@
 // Instantiations of the FP64 blind-rotation kernel for one degree.
 // Compiled once per BR_LOGN (7 .. 12) so the degrees build in parallel.
 #include "br_cluster.cuh"
+#include "br_mma.cuh"
 #include "br_split.cuh"
 #include "br_tm.cuh"
 #include "br_warp.cuh"
@@ -88,6 +89,19 @@ BrKernel TFHE_CAT(br_cluster32_logn, BR_LOGN)(int L, int S) {
     }
     return nullptr;
 }
+#endif
+
+#if BR_LOGN == 10
+BrKernel br_mma_logn10(int L, int M) {
+    if (M != 4 && M != 8) return nullptr;
+    switch (L) {
+        case 2: return M == 8 ? br_mma_kernel<2, 2> : br_mma_kernel<2, 1>;
+        case 3: return M == 8 ? br_mma_kernel<3, 2> : br_mma_kernel<3, 1>;
+        default: return nullptr;
+    }
+}
+
+BmConvKernel bm_key_logn10() { return bm_key_kernel; }
 #endif
 
 #if BR_LOGN == 11

@@ -22,7 +22,8 @@ struct tfhe_keys {
     tfhe_params p;
     int device = -1;
     int G = 0, M = 0;
-    double2* bsk = nullptr;     // [G][2][L][M][N/2][2] FP64 Fourier, position order
+    double2* bsk = nullptr;     // [G][2][L][M][N/2][2] FP64 Fourier, slot order (key_pos)
+    double* bsk_mma = nullptr;  // the same words in br_mma_kernel's layout, where that kernel takes these parameters
     uint32_t* ksk = nullptr;    // [n_big * l_ks][ldk]: columns 0..n-1 mask, n body
     int ldk = 0;
     const tfhe::FftPlan* plan = nullptr;
@@ -598,6 +599,48 @@ static bool persistent_launch(const tfhe_tuning* tune) {
     return (tune && tune->persistent >= 0) ? tune->persistent != 0 : env_on;
 }
 
+// The matrix-instruction kernel (br_mma.cuh) takes N = 1024 on the 32-bit
+// torus, l_bs 2 or 3, four or eight patterns, where the rounded float64
+// products are the exact integers whatever the order of their sums: at
+// log2 beta = 7 (l_bs = 3, eight patterns) a product is at most 0.03 off its
+// integer, and the error grows with beta.
+static bool mma_form(int N, int L, int M, int log2_beta, bool t64, bool reflayout, int kr) {
+    return N == BM_N && !t64 && !reflayout && kr == 0 && log2_beta <= 8 && br_mma_logn10(L, M) != nullptr &&
+           br_mma_smem(L, M) <= (size_t)max_smem_optin();
+}
+
+// Ciphertexts of a batch that go to the matrix-instruction kernel in automatic
+// shapes: whole rounds of four per SM, and the rest too above one per SM
+// (n=630 N=1024, cycles per group and round: this kernel 38k for up to four
+// per SM, the others 22.5k for one, 38.4k for two, 53k for four).
+static long long mma_share(const BrArgs& args, int N, int L, bool reflayout, int kr, const tfhe_tuning* tune) {
+    const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
+    if (!args.bsk_mma || requested || !persistent_launch(tune) ||
+        !mma_form(N, L, args.M, args.log2_beta, args.lwe_a64 != nullptr, reflayout, kr))
+        return 0;
+    const long long sms = std::max(1, sm_count());
+    const long long full = args.B / (BM_K * sms) * (BM_K * sms);
+    return args.B - full > sms ? args.B : full;
+}
+
+static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, const tfhe_tuning* tune) {
+    BrKernel kern = br_mma_logn10(L, args.M);
+    const size_t smem = br_mma_smem(L, args.M);
+    int per_sm = 1;
+    TFHE_TRY(prepare_kernel((const void*)kern, BM_THREADS, smem, &per_sm));
+    BrArgs a = args;
+    const FftPlan* pl = get_plan(N);
+    if (!pl) return TFHE_ERR_INTERNAL;
+    a.qt = pl->qt;
+    a.tw = pl->tw;
+    a.K = BM_K;
+    a.l2_prefetch = (tune && tune->l2_prefetch == 0) ? 0 : 1;
+    const long long sets = (args.B + BM_K - 1) / BM_K;
+    count_launch();
+    kern<<<(unsigned)std::min<long long>(sets, std::max(1, sm_count())), BM_THREADS, smem, stream>>>(a);
+    return check_cuda(cudaGetLastError(), "blind rotation launch (matrix instruction)");
+}
+
 // Ciphertexts of a batch that go to the four-per-CTA kernel in automatic
 // shapes: whole rounds of 4 per SM, and the rest too where a partly filled
 // round is the shortest way (n=742 N=2048, cycles per group and round: four
@@ -651,6 +694,13 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
             if (rest_tune.ciphertexts_per_cta == 3) rest_tune.ciphertexts_per_cta = 0;
             return launch_br(args_after(args, full, N), N, L, reflayout, kr, stream, status, &rest_tune);
         }
+    }
+    if (const long long share = mma_share(args, N, L, reflayout, kr, tune)) {
+        BrArgs head = args;
+        head.B = share;
+        TFHE_TRY(launch_mma(head, N, L, stream, tune));
+        if (share == args.B) return TFHE_OK;
+        return launch_br(args_after(args, share, N), N, L, reflayout, kr, stream, status, tune);
     }
     if (const long long four = warp_four_share(N, L, args.G, args.M, args.B, reflayout, kr, tune)) {
         BrArgs head = args;
@@ -1039,6 +1089,7 @@ static int keys_common(const tfhe_params* params, tfhe_keys** out, tfhe_keys** m
 static void keys_free(tfhe_keys* k) {
     if (!k) return;
     cudaFree(k->bsk);
+    cudaFree(k->bsk_mma);
     cudaFree(k->ksk);
     cudaFree(k->ksk_limbs);
     delete k;
@@ -1047,6 +1098,21 @@ static void keys_free(tfhe_keys* k) {
 static std::atomic<long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 static long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
+
+// the native Fourier key once more in br_mma_kernel's layout, for the
+// parameters that kernel takes
+static int make_mma_key(tfhe_keys* k, cudaStream_t stream) {
+    const tfhe_params& p = k->p;
+    if (!mma_form(p.N, p.l_bs, k->M, p.log2_beta_bs, p.log2_q != 32, false, k->ring_kr)) return TFHE_OK;
+    const size_t bytes = (size_t)4 * k->G * k->M * p.l_bs * (p.N / 2) * sizeof(double2);
+    TFHE_TRY(check_cuda(cudaMalloc(&k->bsk_mma, bytes), "cudaMalloc(bsk, contraction layout)"));
+    k->bytes += (int64_t)bytes;
+    const BmConvArgs ca{k->bsk, k->bsk_mma, k->G, k->M, p.l_bs};
+    count_launch();
+    bm_key_logn10()<<<(unsigned)(std::max(1, sm_count()) * 8), 256, 0, stream>>>(ca);
+    TFHE_TRY(check_cuda(cudaGetLastError(), "bsk layout launch"));
+    return check_cuda(cudaStreamSynchronize(stream), "bsk layout");
+}
 
 // The bootstrapping key (2 in, 2 out, G M, L, N) words of elem bytes (4: the
 // 32-bit torus, 8: the 64-bit one) -> the FP64 Fourier layout the blind
@@ -1149,6 +1215,7 @@ int tfhe_keys_create(const tfhe_params* params, const uint32_t* bsk_coeff, const
     }
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     int rc = upload_bsk(k, bsk_coeff, sizeof(uint32_t), stream);
+    if (rc == TFHE_OK) rc = make_mma_key(k, stream);
     if (rc == TFHE_OK) rc = upload_ksk(k, ksk_a, ksk_b, stream);
     if (rc != TFHE_OK) {
         keys_free(k);
@@ -1208,6 +1275,7 @@ int tfhe_keys_create_fourier(const tfhe_params* params, const double* bsk_ordere
                         "bsk upload");
     }
     if (rc == TFHE_OK) rc = check_cuda(cudaStreamSynchronize(stream), "bsk upload sync");
+    if (rc == TFHE_OK) rc = make_mma_key(k, stream);
     if (rc == TFHE_OK) rc = upload_ksk(k, ksk_a, ksk_b, stream);
     if (rc != TFHE_OK) {
         keys_free(k);
@@ -1301,6 +1369,7 @@ static int br_native(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32_
     if (lut_count != 1 && lut_count != batch) return fail(TFHE_ERR_INVALID_ARGUMENT, "lut_count must be 1 or batch");
     BrArgs a{};
     a.bsk = keys->bsk;
+    a.bsk_mma = keys->bsk_mma;
     a.G = keys->G;
     a.M = keys->M;
     a.collapse = p.collapse;

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "br_cluster.cuh"
+#include "br_mma.cuh"
 #include "br_split.cuh"
 #include "br_tm.cuh"
 #include "br_warp.cuh"
@@ -91,6 +92,12 @@ inline BrKernel br_tm_kernel_for(int logn, int L, bool t64) {
 BrKernel br_warp32_logn11(int NP);
 BrKernel br_warp64_logn11();
 inline BrKernel br_warp_kernel_for(bool t64, int NP) { return t64 ? br_warp64_logn11() : br_warp32_logn11(NP); }
+
+// the matrix-instruction kernels (four ciphertexts per CTA), N = 1024, l_bs 2
+// or 3, four or eight patterns, and their key layout
+using BmConvKernel = void (*)(const BmConvArgs);
+BrKernel br_mma_logn10(int L, int M);
+BmConvKernel bm_key_logn10();
 
 inline BrConvKernel bsk_fft_kernel_for(int logn) {
     switch (logn) {

@@ -56,3 +56,15 @@ def test_n2048_l2_torus64_matches_one_per_cta(collapse):
     keys = Keys64(client64.keygen(p, collapse))
     for i, batch in enumerate(_batches()):
         _compare(keys, p, torch.int64, p.n, batch, (1, 4)[i % 2], 100 * collapse + i)
+
+
+@pytest.mark.parametrize("l_bs,log2_beta,collapse", [(3, 7, 3), (3, 8, 3), (3, 7, 2), (2, 8, 3), (2, 7, 2)])
+def test_n1024_matches_one_per_cta(l_bs, log2_beta, collapse):
+    """The matrix-instruction kernel: its products are the exact integers, so
+    its words are the general kernel's although the sums run in another order."""
+    p = ParamSet("n198_N1024", N=1024, n=198, log2_beta_bs=log2_beta, l_bs=l_bs, collapse=collapse, log2_beta_ks=3,
+                 l_ks=5, sigma_glwe=2.0 ** 7, sigma_lwe=2.0 ** 17)
+    k = client.keygen(p, 10 * l_bs + collapse)
+    keys = Keys.create(p, k.bsk, k.ksk_a, k.ksk_b)
+    for i, batch in enumerate(_batches()):
+        _compare(keys, p, torch.int32, p.n, batch, (1, 4)[i % 2], 100 * collapse + i)
