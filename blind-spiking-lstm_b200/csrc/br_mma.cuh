@@ -117,6 +117,75 @@ __device__ __forceinline__ double bm_rint(double x, double scale) {
     return __dadd_rn(fma(x, scale, MAGIC), -MAGIC);
 }
 
+__device__ __forceinline__ double2 bm_flip(double2 x, uint32_t sign) {
+    return make_double2(__hiloint2double(__double2hiint(x.x) ^ (int)sign, __double2loint(x.x)),
+                        __hiloint2double(__double2hiint(x.y) ^ (int)sign, __double2loint(x.y)));
+}
+
+// X^r at the four points p .. p + 3 (p a multiple of 4) for the lane's pattern
+// of every tile: the points' frequencies (the position's bits reversed) differ
+// by half (bit 0) and a quarter (bit 1) of the circle, so one read of the
+// half-circle table gives all four, w[t][bit 1], times (-1)^r for bit 0
+template <int T>
+__device__ __forceinline__ void bm_twist(double2 (&w)[T][2], const int (&r)[T], const double2* hc, int p) {
+    const int e = 4 * (int)(__brev((unsigned)p) >> 23) + 1;          // the point zeta^e, H = 512
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        const int idx = r[t] * e;
+        const double2 x = bm_flip(hc[idx & (BM_N - 1)], (uint32_t)(idx << 21) & 0x80000000u);
+        const double2 y = (r[t] & 1) ? c_mul_mi(x) : x;              // times (-i)^r
+        w[t][0] = x;
+        w[t][1] = bm_flip(y, (uint32_t)(r[t] << 30) & 0x80000000u);
+    }
+}
+
+// T = key x digits of four points (2 T sums side by side: an instruction's
+// result takes 28 cycles, its issue 16); reload(h) once the key words of pair
+// h are consumed
+template <int L, int T, class Reload>
+__device__ __forceinline__ void bm_products(double (&c)[4][T][2], double2 (&ka)[T][L], double2 (&kb)[T][L],
+                                            const double (&b)[4][L], Reload reload) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int s = 0; s < L; ++s)
+#pragma unroll
+            for (int i = 2 * h; i < 2 * h + 2; ++i)
+#pragma unroll
+                for (int t = 0; t < T; ++t) {
+                    if (s == 0) c[i][t][0] = c[i][t][1] = 0.0;
+                    const double2 k2 = h == 0 ? ka[t][s] : kb[t][s];
+                    bm_mma(c[i][t], (i & 1) == 0 ? k2.x : k2.y, b[i][s]);
+                }
+        reload(h);
+    }
+}
+
+// the four points' outputs from T: times X^r, summed over the tiles in the
+// lane and over the four rows of a tile (lane bits 2 and 3); y[j] is then
+// component bit 2 of point 2 j + bit 3
+template <int T>
+__device__ __forceinline__ void bm_sums(double (&y)[2], const double (&c)[4][T][2], const double2 (&w)[T][2],
+                                        const int (&r)[T], int lane) {
+    const bool b2 = lane & 4, b3 = lane & 8;
+    double x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        double2 o;
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            const double2 f = (i & 1) ? bm_flip(w[t][i >> 1], (uint32_t)r[t] << 31) : w[t][i >> 1];
+            if (t == 0) o = make_double2(f.x * c[i][t][0], f.x * c[i][t][1]);
+            else o = make_double2(fma(f.x, c[i][t][0], o.x), fma(f.x, c[i][t][1], o.y));
+            o.x = fma(-f.y, c[i][t][1], o.x);
+            o.y = fma(f.y, c[i][t][0], o.y);
+        }
+        x[i] = (b2 ? o.y : o.x) + bm_shfl(b2 ? o.x : o.y, 4);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) y[j] = (b3 ? x[2 * j + 1] : x[2 * j]) + bm_shfl(b3 ? x[2 * j] : x[2 * j + 1], 8);
+}
+
 // Double of the contraction layout: group g, warp w, pair u of its points
 // (point w 32 + 2 u + sl), tile t, digit pair s, lane (row o 4 + mm, k), sl
 __host__ __device__ __forceinline__ size_t bm_key_at(int L, int T, size_t g, int w, int u, int t, int s, int lane,
@@ -324,49 +393,12 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_kernel(const BrArgs args
                 const double* bbase = reinterpret_cast<const double*>(dec + (bk * P + bdig) * H) + bcomp;
                 const int bx = bk * 2 + bdig;                        // bm_at's exclusive-or of this lane's digits
                 const int p0 = warp * 32;
-                // X^r at the four points 4 v .. 4 v + 3: their frequencies differ by
-                // half (bit 0) and a quarter (bit 1) of the circle, so one table
-                // read gives all four: times (-1)^r and (-i)^r
-                double2 w[T][2];
-                uint32_t odd[T];
-#pragma unroll
-                for (int t = 0; t < T; ++t) odd[t] = (uint32_t)rr[t] << 31;
-                auto flip = [](double2 x, uint32_t sg) {
-                    return make_double2(__hiloint2double(__double2hiint(x.x) ^ (int)sg, __double2loint(x.x)),
-                                        __hiloint2double(__double2hiint(x.y) ^ (int)sg, __double2loint(x.y)));
-                };
-                auto twist = [&](int v) {
-                    const int e = 4 * (int)(__brev((unsigned)(p0 + 4 * v)) >> (32 - LOGH)) + 1;
-#pragma unroll
-                    for (int t = 0; t < T; ++t) {
-                        const int idx = rr[t] * e;
-                        const double2 x = flip(hc[idx & (N - 1)], (uint32_t)(idx << (31 - LOGN)) & 0x80000000u);
-                        w[t][0] = x;
-                        // times (-i)^r
-                        const double2 y = (rr[t] & 1) ? c_mul_mi(x) : x;
-                        w[t][1] = flip(y, (uint32_t)(rr[t] << 30) & 0x80000000u);
-                    }
-                };
-                // sum over the patterns of the lane's tiles
-                auto twisted = [&](const double (&c)[T][2], int sl, int hf) {
-                    double2 o;
-#pragma unroll
-                    for (int t = 0; t < T; ++t) {
-                        const double2 x = sl == 0 ? w[t][hf] : flip(w[t][hf], odd[t]);
-                        if (t == 0) o = make_double2(x.x * c[t][0], x.x * c[t][1]);
-                        else o = make_double2(fma(x.x, c[t][0], o.x), fma(x.x, c[t][1], o.y));
-                        o.x = fma(-x.y, c[t][1], o.x);
-                        o.y = fma(x.y, c[t][0], o.y);
-                    }
-                    return o;
-                };
-                const bool b2 = lane & 4, b3 = lane & 8;
                 load(ka, 0);
                 load(kb, 1);
 #pragma unroll 1
                 for (int u = 0; u < 16; u += 2) {
-                    double c[4][T][2];
-                    double b[4][L];
+                    double c[4][T][2], b[4][L], y[2];
+                    double2 w[T][2];
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -375,37 +407,17 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_kernel(const BrArgs args
                             const double x = bbase[(size_t)(2 * s * H + (p ^ ((p >> 3) & 7) ^ bx)) * 2];
                             b[i][s] = __hiloint2double(__double2hiint(x) ^ bsign, __double2loint(x));
                         }
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                        for (int s = 0; s < L; ++s)
-#pragma unroll
-                            for (int i = 2 * h; i < 2 * h + 2; ++i)
-#pragma unroll
-                                for (int t = 0; t < T; ++t) {
-                                    if (s == 0) c[i][t][0] = c[i][t][1] = 0.0;
-                                    const double2 k2 = h == 0 ? ka[t][s] : kb[t][s];
-                                    bm_mma(c[i][t], (i & 1) == 0 ? k2.x : k2.y, b[i][s]);
-                                }
+                    bm_products<L, T>(c, ka, kb, b, [&](int h) {
                         if (u < 14) {
                             if (h == 0) load(ka, u + 2);
                             else load(kb, u + 3);
                         }
-                    }
-                    twist(u >> 1);
-                    double2 o[4];
+                    });
+                    bm_twist<T>(w, rr, hc, p0 + 2 * u);
+                    bm_sums<T>(y, c, w, rr, lane);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) o[i] = twisted(c[i], i & 1, i >> 1);
-                    // sum over the four rows (lane bits 2 and 3): bit 2 then names the
-                    // component, bit 3 the point of a pair
-                    double x[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) x[i] = (b2 ? o[i].y : o[i].x) + bm_shfl(b2 ? o[i].x : o[i].y, 4);
-#pragma unroll
-                    for (int i = 0; i < 4; i += 2) {
-                        const double y = (b3 ? x[i + 1] : x[i]) + bm_shfl(b3 ? x[i] : x[i + 1], 8);
-                        reinterpret_cast<double*>(dec + bm_at<P>(tk, to, p0 + 2 * u + i + (b3 ? 1 : 0)))[b2 ? 1 : 0] = y;
-                    }
+                    for (int j = 0; j < 2; ++j)
+                        reinterpret_cast<double*>(dec + bm_at<P>(tk, to, p0 + 2 * (u + j) + ((lane >> 3) & 1)))[(lane >> 2) & 1] = y[j];
                 }
             }
             bm_pair_barrier(bar_id);

@@ -387,8 +387,8 @@ static bool split_enabled() {
     return on;
 }
 
-// one ciphertext per cluster of `csize` CTAs: grid csize * B
-static int launch_cluster(BrKernel kern, int nt, size_t smem, int csize, const BrArgs& args, int N,
+// `clusters` clusters of `csize` CTAs
+static int launch_cluster(BrKernel kern, int nt, size_t smem, int csize, long long clusters, const BrArgs& args, int N,
                           cudaStream_t stream, const tfhe_tuning* tune, const char* what) {
     int per_sm = 1;
     TFHE_TRY(prepare_kernel((const void*)kern, nt, smem, &per_sm));
@@ -401,8 +401,11 @@ static int launch_cluster(BrKernel kern, int nt, size_t smem, int csize, const B
     a.freq = pl->freq;
     a.K = 1;
     a.l2_prefetch = (tune && tune->l2_prefetch == 0) ? 0 : 1;
+    a.wait_limit = WAIT_LIMIT_CYCLES;
+    a.status = device_status_word();
+    if (!a.status) return fail(TFHE_ERR_INTERNAL, "device status word unavailable");
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(csize * args.B), 1, 1);
+    cfg.gridDim = dim3((unsigned)(csize * clusters), 1, 1);
     cfg.blockDim = dim3(nt, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -421,8 +424,8 @@ static int launch_split(const BrArgs& args, int N, int L, cudaStream_t stream, c
     const bool t64 = args.lwe_a64 != nullptr;
     BrKernel kern = br_split_kernel_for(ilog2(N), L, t64);
     if (!kern) return fail(TFHE_ERR_INVALID_ARGUMENT, "unsupported degree / levels");
-    return launch_cluster(kern, BR_SPLIT_THREADS, br_split_smem(N, L, args.G, args.M, br_table_bytes(N)), 2, args, N,
-                          stream, tune, "blind rotation launch (cluster pair)");
+    return launch_cluster(kern, BR_SPLIT_THREADS, br_split_smem(N, L, args.G, args.M, br_table_bytes(N)), 2, args.B,
+                          args, N, stream, tune, "blind rotation launch (cluster pair)");
 }
 
 // one ciphertext per cluster of 2 S CTAs (br_cluster.cuh)
@@ -431,7 +434,7 @@ static int launch_cluster_s(const BrArgs& args, int N, int L, int S, cudaStream_
     BrKernel kern = br_cluster_kernel_for(ilog2(N), L, t64, S);
     if (!kern) return fail(TFHE_ERR_INVALID_ARGUMENT, "unsupported degree / levels");
     return launch_cluster(kern, BR_CLUSTER_THREADS, br_cluster_smem(N, L, args.G, args.M, br_table_bytes(N), S),
-                          2 * S, args, N, stream, tune,
+                          2 * S, args.B, args, N, stream, tune,
                           S == 4 ? "blind rotation launch (cluster of eight)" : "blind rotation launch (cluster of four)");
 }
 
@@ -609,18 +612,24 @@ static bool mma_form(int N, int L, int M, int log2_beta, bool t64, bool reflayou
            br_mma_smem(L, M) <= (size_t)max_smem_optin();
 }
 
-// Ciphertexts of a batch that go to the matrix-instruction kernel in automatic
-// shapes: whole rounds of four per SM, and the rest too above one per SM
-// (n=630 N=1024, cycles per group and round: this kernel 38k for up to four
-// per SM, the others 22.5k for one, 38.4k for two, 53k for four).
-static long long mma_share(const BrArgs& args, int N, int L, bool reflayout, int kr, const tfhe_tuning* tune) {
+// The matrix-instruction kernels take this launch: automatic shapes of keys in
+// their layout.
+static bool mma_takes(const BrArgs& args, int N, int L, bool reflayout, int kr, const tfhe_tuning* tune) {
     const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
-    if (!args.bsk_mma || requested || !persistent_launch(tune) ||
-        !mma_form(N, L, args.M, args.log2_beta, args.lwe_a64 != nullptr, reflayout, kr))
-        return 0;
-    const long long sms = std::max(1, sm_count());
-    const long long full = args.B / (BM_K * sms) * (BM_K * sms);
-    return args.B - full > sms ? args.B : full;
+    return args.bsk_mma && !requested && persistent_launch(tune) &&
+           mma_form(N, L, args.M, args.log2_beta, args.lwe_a64 != nullptr, reflayout, kr);
+}
+
+// ciphertexts that one wave of clusters of C CTAs takes, four per cluster
+static long long mma_cluster_capacity(int L, int M, int C) {
+    if (!split_enabled() || (C >= 4 && !quad_enabled()) || (C == 8 && !octet_enabled())) return 0;
+    return BM_K * resident_clusters(br_mma_cluster_logn10(L, M, C), BM_THREADS, br_mma_cluster_smem_for(L, M, C), C);
+}
+
+static int launch_mma_cluster(const BrArgs& args, int N, int L, int C, cudaStream_t stream, const tfhe_tuning* tune) {
+    return launch_cluster(br_mma_cluster_logn10(L, args.M, C), BM_THREADS, br_mma_cluster_smem_for(L, args.M, C), C,
+                          (args.B + BM_K - 1) / BM_K, args, N, stream, tune,
+                          "blind rotation launch (matrix instruction, cluster)");
 }
 
 static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, const tfhe_tuning* tune) {
@@ -678,6 +687,20 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
                      int* status = nullptr, const tfhe_tuning* tune = nullptr) {
     const int logn = ilog2(N);
     const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
+    if (mma_takes(args, N, L, reflayout, kr, tune)) {
+        // whole rounds of four per SM, then the rest on the widest clusters
+        // that hold it in one wave, or a partly filled round
+        const long long round = (long long)BM_K * std::max(1, sm_count());
+        const long long full = args.B / round * round;
+        const long long rest = args.B - full;
+        int C = 0;
+        for (int c : {2, 4, 8})
+            if (rest > 0 && rest <= mma_cluster_capacity(L, args.M, c)) C = c;
+        BrArgs head = args;
+        head.B = C ? full : args.B;
+        if (head.B > 0) TFHE_TRY(launch_mma(head, N, L, stream, tune));
+        return C ? launch_mma_cluster(full ? args_after(args, full, N) : args, N, L, C, stream, tune) : TFHE_OK;
+    }
     if (const int S = cluster_form(N, L, args.G, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
         return launch_cluster_s(args, N, L, S, stream, tune);
     if (split_applies(N, L, args.G, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
@@ -694,13 +717,6 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
             if (rest_tune.ciphertexts_per_cta == 3) rest_tune.ciphertexts_per_cta = 0;
             return launch_br(args_after(args, full, N), N, L, reflayout, kr, stream, status, &rest_tune);
         }
-    }
-    if (const long long share = mma_share(args, N, L, reflayout, kr, tune)) {
-        BrArgs head = args;
-        head.B = share;
-        TFHE_TRY(launch_mma(head, N, L, stream, tune));
-        if (share == args.B) return TFHE_OK;
-        return launch_br(args_after(args, share, N), N, L, reflayout, kr, stream, status, tune);
     }
     if (const long long four = warp_four_share(N, L, args.G, args.M, args.B, reflayout, kr, tune)) {
         BrArgs head = args;

@@ -4,6 +4,7 @@
 
 #include "br_cluster.cuh"
 #include "br_mma.cuh"
+#include "br_mma_cluster.cuh"
 #include "br_split.cuh"
 #include "br_tm.cuh"
 #include "br_warp.cuh"
@@ -97,6 +98,9 @@ inline BrKernel br_warp_kernel_for(bool t64, int NP) { return t64 ? br_warp64_lo
 // or 3, four or eight patterns, and their key layout
 using BmConvKernel = void (*)(const BmConvArgs);
 BrKernel br_mma_logn10(int L, int M);
+// the same on clusters of C = 2, 4 or 8 CTAs for four ciphertexts
+BrKernel br_mma_cluster_logn10(int L, int M, int C);
+size_t br_mma_cluster_smem_for(int L, int M, int C);
 BmConvKernel bm_key_logn10();
 
 inline BrConvKernel bsk_fft_kernel_for(int logn) {

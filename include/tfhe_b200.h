@@ -131,8 +131,10 @@ int tfhe_keys_launch_shape(const tfhe_keys* keys, int64_t batch, int32_t* cipher
  * or 2048, at most a quarter;
  * TFHE_B200_QUAD=0 turns both off), 2 on a cluster of two (at most half the
  * SM count), else 1 (automatic shapes only; TFHE_B200_SPLIT=0 turns every
- * cluster form off); 0 for NULL keys.  Speed only: every form gives
- * identical outputs. */
+ * cluster form off); 0 for NULL keys.  At N = 1024, gadget base <= 2^8, l_bs 2
+ * or 3 and collapse 2 or 3 the matrix-instruction form takes these batches
+ * instead, four ciphertexts per cluster of eight, four or two CTAs (the same
+ * switches turn those off).  Speed only: every form gives identical outputs. */
 int32_t tfhe_keys_cluster_size(const tfhe_keys* keys, int64_t batch);
 int64_t tfhe_keys_device_bytes(const tfhe_keys* keys);
 

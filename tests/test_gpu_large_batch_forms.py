@@ -66,5 +66,8 @@ def test_n1024_matches_one_per_cta(l_bs, log2_beta, collapse):
                  l_ks=5, sigma_glwe=2.0 ** 7, sigma_lwe=2.0 ** 17)
     k = client.keygen(p, 10 * l_bs + collapse)
     keys = Keys.create(p, k.bsk, k.ksk_a, k.ksk_b)
-    for i, batch in enumerate(_batches()):
+    # below a round: clusters of eight, four and two CTAs for four ciphertexts
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    small = [1, 3, 4, 5, sms // 4, sms // 2, sms // 2 + 1, sms - 20, sms]
+    for i, batch in enumerate(small + _batches()):
         _compare(keys, p, torch.int32, p.n, batch, (1, 4)[i % 2], 100 * collapse + i)
