@@ -1,8 +1,6 @@
 // Instantiations of the FP64 blind-rotation kernel for one degree.
 // Compiled once per BR_LOGN (7 .. 12) so the degrees build in parallel.
 #include "br_cluster.cuh"
-#include "br_mma.cuh"
-#include "br_mma_cluster.cuh"
 #include "br_split.cuh"
 #include "br_tm.cuh"
 #include "br_warp.cuh"
@@ -90,37 +88,6 @@ BrKernel TFHE_CAT(br_cluster32_logn, BR_LOGN)(int L, int S) {
     }
     return nullptr;
 }
-#endif
-
-#if BR_LOGN == 10
-BrKernel br_mma_logn10(int L, int M) {
-    if (M != 4 && M != 8) return nullptr;
-    switch (L) {
-        case 2: return M == 8 ? br_mma_kernel<2, 2> : br_mma_kernel<2, 1>;
-        case 3: return M == 8 ? br_mma_kernel<3, 2> : br_mma_kernel<3, 1>;
-        default: return nullptr;
-    }
-}
-
-template <int L, int T>
-static BrKernel mma_cluster_of(int C) {
-    return C == 2 ? br_mma_cluster_kernel<L, T, 2> : C == 4 ? br_mma_cluster_kernel<L, T, 4>
-         : C == 8 ? br_mma_cluster_kernel<L, T, 8> : nullptr;
-}
-
-BrKernel br_mma_cluster_logn10(int L, int M, int C) {
-    if (M != 4 && M != 8) return nullptr;
-    if (L == 2) return M == 8 ? mma_cluster_of<2, 2>(C) : mma_cluster_of<2, 1>(C);
-    if (L == 3) return M == 8 ? mma_cluster_of<3, 2>(C) : mma_cluster_of<3, 1>(C);
-    return nullptr;
-}
-
-size_t br_mma_cluster_smem_for(int L, int M, int C) {
-    if (L == 2) return C == 2 ? br_mma_cluster_smem<2, 2>(M) : C == 4 ? br_mma_cluster_smem<2, 4>(M) : br_mma_cluster_smem<2, 8>(M);
-    return C == 2 ? br_mma_cluster_smem<3, 2>(M) : C == 4 ? br_mma_cluster_smem<3, 4>(M) : br_mma_cluster_smem<3, 8>(M);
-}
-
-BmConvKernel bm_key_logn10() { return bm_key_kernel; }
 #endif
 
 #if BR_LOGN == 11

@@ -224,7 +224,46 @@ static __global__ void __launch_bounds__(256) bm_key_kernel(const BmConvArgs a) 
     }
 }
 
-template <int L, int T>
+// the reference's key (G, 2 out, L, 2 in, M, H) at zeta^(2 j + 1), j < H ->
+// contraction layout: the same points or their conjugate partners, times 1/H
+// as the native key is stored (a power of two, so exact).  One block per
+// (group, output, level, pattern); reads whole rows, writes 64 bytes in a row.
+struct BmRefConvArgs {
+    const double2* src;
+    double* dst;
+    int M, L;
+};
+
+static __global__ void __launch_bounds__(256) bm_ref_key_kernel(const BmRefConvArgs a) {
+    __shared__ double2 row[2][BM_H];
+    const int T = a.M / 4;
+    const int m = blockIdx.x % a.M;
+    int r = blockIdx.x / a.M;
+    const int s = r % a.L;
+    r /= a.L;
+    const int o = r & 1;
+    const size_t g = r >> 1;
+    for (int i = threadIdx.x; i < 2 * BM_H; i += 256) {
+        const int in = i / BM_H, j = i % BM_H;
+        row[in][j] = a.src[(((((g * 2 + o) * a.L + s) * 2 + in) * a.M) + m) * BM_H + j];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 4 * (BM_H / 2); i += 256) {
+        const int k = i & 3, pu = i >> 2;                            // k: digit's (re, im); pair of points
+        double v[2];
+#pragma unroll
+        for (int sl = 0; sl < 2; ++sl) {
+            const int j = (int)(__brev((unsigned)(2 * pu + sl)) >> 23), e = 4 * j + 1;
+            const double2 z = e < BM_N ? row[k >> 1][2 * j] : c_conj(row[k >> 1][BM_N - 1 - 2 * j]);
+            v[sl] = ((k & 1) ? z.y : z.x) * (1.0 / BM_H);
+        }
+        const size_t at = bm_key_at(a.L, T, g, pu >> 4, pu & 15, m >> 2, s, (o * 4 + (m & 3)) * 4 + k, 0);
+        *reinterpret_cast<double2*>(a.dst + at) = make_double2(v[0], v[1]);
+    }
+}
+
+// REF: the drop-in's inputs and outputs (int64 accumulators, indices given)
+template <int L, int T, bool REF>
 __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_kernel(const BrArgs args) {
     constexpr int LOGN = 10, LOGH = 9, P = 2 * L, K = BM_K, M = 4 * T;
     constexpr int N = BM_N, H = BM_H;
@@ -283,11 +322,20 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_kernel(const BrArgs args
         double acc_lo[8], acc_hi[8];
         {
             const long long oct = min(ct0 + ok, args.B - 1);
-            const uint32_t* src = args.lut + oct * args.lut_stride + oa * N;
+            if constexpr (REF) {
+                const int64_t* src = args.ct_init + oct * args.ct_stride + oa * N;
 #pragma unroll
-            for (int n = 0; n < 8; ++n) {
-                acc_lo[n] = (double)(int32_t)src[oc + 64 * n];
-                acc_hi[n] = (double)(int32_t)src[oc + 64 * n + H];
+                for (int n = 0; n < 8; ++n) {
+                    acc_lo[n] = (double)src[oc + 64 * n];
+                    acc_hi[n] = (double)src[oc + 64 * n + H];
+                }
+            } else {
+                const uint32_t* src = args.lut + oct * args.lut_stride + oa * N;
+#pragma unroll
+                for (int n = 0; n < 8; ++n) {
+                    acc_lo[n] = (double)(int32_t)src[oc + 64 * n];
+                    acc_hi[n] = (double)(int32_t)src[oc + 64 * n + H];
+                }
             }
         }
         __syncthreads();
@@ -311,6 +359,10 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_kernel(const BrArgs args
                 for (int x = tid; x < ng * K * M; x += BM_THREADS) {
                     const int gg = x / (K * M), k = (x / M) % K, m = x % M;
                     const long long ct = min(ct0 + k, args.B - 1);
+                    if constexpr (REF) {
+                        rot[x] = (uint16_t)(args.indices[(ct * args.G + g + gg) * M + m] & (2 * N - 1));
+                        continue;
+                    }
                     double v = 0.0;
                     const uint32_t* a = args.lwe_a + ct * args.lwe_n + (long long)(g + gg) * args.collapse;
                     for (int c = 0; c < args.collapse; ++c)
@@ -468,6 +520,17 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_kernel(const BrArgs args
         }
         __syncthreads();                                             // dec is reused below
 
+        if constexpr (REF) {
+            if (ct0 + ok < args.B) {
+                int64_t* dst = args.out_i64 + (ct0 + ok) * 2 * N + oa * N;
+#pragma unroll
+                for (int n = 0; n < 8; ++n) {
+                    dst[oc + 64 * n] = __double2ll_rn(acc_lo[n]);
+                    dst[oc + 64 * n + H] = __double2ll_rn(acc_hi[n]);
+                }
+            }
+            continue;
+        }
         // epilogue: rotate by -b~ and extract, as br_fp64_kernel
         uint32_t* acc = reinterpret_cast<uint32_t*>(smem_raw);       // [K][2][N]
         {

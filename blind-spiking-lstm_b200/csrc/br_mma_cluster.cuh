@@ -117,7 +117,7 @@ __device__ __forceinline__ void bmc_wait(uint64_t* bar, uint32_t parity, long lo
     }
 }
 
-template <int L, int T, int C>
+template <int L, int T, int C, bool REF>
 __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrArgs args) {
     using S = BmcShape<L, C>;
     constexpr int LOGN = 10, LOGH = 9, P = 2 * L, K = BM_K, M = 4 * T;
@@ -238,11 +238,20 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
         double acc_lo[8], acc_hi[8];
         {
             const long long oct = min(ct0 + ct_in, args.B - 1);
-            const uint32_t* src = args.lut + oct * args.lut_stride + oa * N;
+            if constexpr (REF) {
+                const int64_t* src = args.ct_init + oct * args.ct_stride + oa * N;
 #pragma unroll
-            for (int n = 0; n < 8; ++n) {
-                acc_lo[n] = (double)(int32_t)src[oc + 64 * n];
-                acc_hi[n] = (double)(int32_t)src[oc + 64 * n + H];
+                for (int n = 0; n < 8; ++n) {
+                    acc_lo[n] = (double)src[oc + 64 * n];
+                    acc_hi[n] = (double)src[oc + 64 * n + H];
+                }
+            } else {
+                const uint32_t* src = args.lut + oct * args.lut_stride + oa * N;
+#pragma unroll
+                for (int n = 0; n < 8; ++n) {
+                    acc_lo[n] = (double)(int32_t)src[oc + 64 * n];
+                    acc_hi[n] = (double)(int32_t)src[oc + 64 * n + H];
+                }
             }
         }
         copy(0);
@@ -270,6 +279,10 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
                 for (int x = tid; x < ng * K * M; x += BM_THREADS) {
                     const int gg = x / (K * M), k = (x / M) % K, m = x % M;
                     const long long ct = min(ct0 + k, args.B - 1);
+                    if constexpr (REF) {
+                        rot[x] = (uint16_t)(args.indices[(ct * args.G + g + gg) * M + m] & (2 * N - 1));
+                        continue;
+                    }
                     double v = 0.0;
                     const uint32_t* a = args.lwe_a + ct * args.lwe_n + (long long)(g + gg) * args.collapse;
                     for (int c = 0; c < args.collapse; ++c)
@@ -475,6 +488,17 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
         }
         __syncthreads();                                             // dig and out are reused below
 
+        if constexpr (REF) {
+            if (owner && (!S::LP || olv == 0) && ct0 + ct_in < args.B) {
+                int64_t* dst = args.out_i64 + (ct0 + ct_in) * 2 * N + oa * N;
+#pragma unroll
+                for (int n = 0; n < 8; ++n) {
+                    dst[oc + 64 * n] = __double2ll_rn(acc_lo[n]);
+                    dst[oc + 64 * n + H] = __double2ll_rn(acc_hi[n]);
+                }
+            }
+            continue;
+        }
         // epilogue: rotate by -b~ and extract, as br_fp64_kernel; C = 8: the
         // CTA of polynomial 0 the masks, that of polynomial 1 the bodies
         uint32_t* acc = reinterpret_cast<uint32_t*>(smem_raw);       // [NA][N]

@@ -144,6 +144,46 @@ int* device_status_word() {
     return w;
 }
 
+// Working memory comes from a pool of the library's own per device that keeps
+// up to SCRATCH_KEEP bytes over a synchronisation.  The device's default pool
+// keeps none: each first call after one paid for mapping its memory again
+// (0.5 to 1 ms for a small bootstrap, 2 ms for the drop-in's 165 MB).  The kept
+// memory goes back when a key set is destroyed, and at exit.
+constexpr uint64_t SCRATCH_KEEP = 256ull << 20;
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pool[64];
+
+static cudaMemPool_t scratch_pool(int dev) {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        uint64_t keep = SCRATCH_KEEP;
+        if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+            if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) g_pool[dev] = pool;
+            else cudaMemPoolDestroy(pool);
+        }
+        cudaGetLastError();
+    }
+    return g_pool[dev];
+}
+
+cudaError_t scratch_alloc(void** out, size_t bytes, cudaStream_t stream) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaMemPool_t pool = dev >= 0 && dev < 64 ? scratch_pool(dev) : nullptr;
+    return pool ? cudaMallocFromPoolAsync(out, bytes, pool, stream) : cudaMallocAsync(out, bytes, stream);
+}
+
+static void scratch_trim(int dev) {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (dev >= 0 && dev < 64 && g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
+}
+
 const FftPlan* get_plan(int N) {
     int dev = 0;
     if (check_cuda(cudaGetDevice(&dev), "cudaGetDevice") != TFHE_OK) return nullptr;
@@ -602,52 +642,64 @@ static bool persistent_launch(const tfhe_tuning* tune) {
     return (tune && tune->persistent >= 0) ? tune->persistent != 0 : env_on;
 }
 
-// The matrix-instruction kernel (br_mma.cuh) takes N = 1024 on the 32-bit
-// torus, l_bs 2 or 3, four or eight patterns, where the rounded float64
-// products are the exact integers whatever the order of their sums: at
+// The matrix-instruction kernels (br_mma.cuh, br_mma_cluster.cuh) take N = 1024
+// on the 32-bit torus, l_bs 2 or 3, four or eight patterns, where the rounded
+// float64 products are the exact integers whatever the order of their sums: at
 // log2 beta = 7 (l_bs = 3, eight patterns) a product is at most 0.03 off its
 // integer, and the error grows with beta.
-static bool mma_form(int N, int L, int M, int log2_beta, bool t64, bool reflayout, int kr) {
-    return N == BM_N && !t64 && !reflayout && kr == 0 && log2_beta <= 8 && br_mma_logn10(L, M) != nullptr &&
-           br_mma_smem(L, M) <= (size_t)max_smem_optin();
+static bool mma_form(int N, int L, int M, int log2_beta, int log2_q) {
+    return N == BM_N && log2_q == 32 && log2_beta <= 8 && (L == 2 || L == 3) && (M == 4 || M == 8) &&
+           br_mma_smem_for(L, M, 1) <= (size_t)max_smem_optin();
 }
 
-// The matrix-instruction kernels take this launch: automatic shapes of keys in
-// their layout.
-static bool mma_takes(const BrArgs& args, int N, int L, bool reflayout, int kr, const tfhe_tuning* tune) {
+// this launch: automatic shapes of keys in their layout
+static bool mma_takes(const BrArgs& args, int N, int L, const tfhe_tuning* tune) {
     const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
     return args.bsk_mma && !requested && persistent_launch(tune) &&
-           mma_form(N, L, args.M, args.log2_beta, args.lwe_a64 != nullptr, reflayout, kr);
+           mma_form(N, L, args.M, args.log2_beta, args.log2_q);
 }
 
 // ciphertexts that one wave of clusters of C CTAs takes, four per cluster
-static long long mma_cluster_capacity(int L, int M, int C) {
+static long long mma_cluster_capacity(int L, int M, int C, bool ref) {
     if (!split_enabled() || (C >= 4 && !quad_enabled()) || (C == 8 && !octet_enabled())) return 0;
-    return BM_K * resident_clusters(br_mma_cluster_logn10(L, M, C), BM_THREADS, br_mma_cluster_smem_for(L, M, C), C);
+    return BM_K * resident_clusters(br_mma_kernel_for(L, M, C, ref), BM_THREADS, br_mma_smem_for(L, M, C), C);
 }
 
-static int launch_mma_cluster(const BrArgs& args, int N, int L, int C, cudaStream_t stream, const tfhe_tuning* tune) {
-    return launch_cluster(br_mma_cluster_logn10(L, args.M, C), BM_THREADS, br_mma_cluster_smem_for(L, args.M, C), C,
-                          (args.B + BM_K - 1) / BM_K, args, N, stream, tune,
-                          "blind rotation launch (matrix instruction, cluster)");
-}
-
+// Whole rounds of four ciphertexts per SM, then the rest on the widest clusters
+// that hold it in one wave, or a partly filled round (n=630, cycles per group:
+// four per SM 38k, clusters of two 27k for two per SM, of four 18.5k for about
+// one per SM, of eight 11.3k).
 static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, const tfhe_tuning* tune) {
-    BrKernel kern = br_mma_logn10(L, args.M);
-    const size_t smem = br_mma_smem(L, args.M);
-    int per_sm = 1;
-    TFHE_TRY(prepare_kernel((const void*)kern, BM_THREADS, smem, &per_sm));
-    BrArgs a = args;
-    const FftPlan* pl = get_plan(N);
-    if (!pl) return TFHE_ERR_INTERNAL;
-    a.qt = pl->qt;
-    a.tw = pl->tw;
-    a.K = BM_K;
-    a.l2_prefetch = (tune && tune->l2_prefetch == 0) ? 0 : 1;
-    const long long sets = (args.B + BM_K - 1) / BM_K;
-    count_launch();
-    kern<<<(unsigned)std::min<long long>(sets, std::max(1, sm_count())), BM_THREADS, smem, stream>>>(a);
-    return check_cuda(cudaGetLastError(), "blind rotation launch (matrix instruction)");
+    const bool ref = args.ct_init != nullptr;
+    const long long round = (long long)BM_K * std::max(1, sm_count());
+    const long long full = args.B / round * round;
+    const long long rest = args.B - full;
+    int C = 0;
+    for (int c : {2, 4, 8})
+        if (rest > 0 && rest <= mma_cluster_capacity(L, args.M, c, ref)) C = c;
+    const long long head = C ? full : args.B;
+    if (head > 0) {
+        BrKernel kern = br_mma_kernel_for(L, args.M, 1, ref);
+        const size_t smem = br_mma_smem_for(L, args.M, 1);
+        int per_sm = 1;
+        TFHE_TRY(prepare_kernel((const void*)kern, BM_THREADS, smem, &per_sm));
+        const FftPlan* pl = get_plan(N);
+        if (!pl) return TFHE_ERR_INTERNAL;
+        BrArgs a = args;
+        a.qt = pl->qt;
+        a.tw = pl->tw;
+        a.K = BM_K;
+        a.B = head;
+        a.l2_prefetch = (tune && tune->l2_prefetch == 0) ? 0 : 1;
+        const long long sets = (head + BM_K - 1) / BM_K;
+        count_launch();
+        kern<<<(unsigned)std::min<long long>(sets, std::max(1, sm_count())), BM_THREADS, smem, stream>>>(a);
+        TFHE_TRY(check_cuda(cudaGetLastError(), "blind rotation launch (matrix instruction)"));
+    }
+    if (!C) return TFHE_OK;
+    return launch_cluster(br_mma_kernel_for(L, args.M, C, ref), BM_THREADS, br_mma_smem_for(L, args.M, C), C,
+                          (rest + BM_K - 1) / BM_K, full ? args_after(args, full, N) : args, N, stream, tune,
+                          "blind rotation launch (matrix instruction, cluster)");
 }
 
 // Ciphertexts of a batch that go to the four-per-CTA kernel in automatic
@@ -687,20 +739,7 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
                      int* status = nullptr, const tfhe_tuning* tune = nullptr) {
     const int logn = ilog2(N);
     const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
-    if (mma_takes(args, N, L, reflayout, kr, tune)) {
-        // whole rounds of four per SM, then the rest on the widest clusters
-        // that hold it in one wave, or a partly filled round
-        const long long round = (long long)BM_K * std::max(1, sm_count());
-        const long long full = args.B / round * round;
-        const long long rest = args.B - full;
-        int C = 0;
-        for (int c : {2, 4, 8})
-            if (rest > 0 && rest <= mma_cluster_capacity(L, args.M, c)) C = c;
-        BrArgs head = args;
-        head.B = C ? full : args.B;
-        if (head.B > 0) TFHE_TRY(launch_mma(head, N, L, stream, tune));
-        return C ? launch_mma_cluster(full ? args_after(args, full, N) : args, N, L, C, stream, tune) : TFHE_OK;
-    }
+    if (mma_takes(args, N, L, tune)) return launch_mma(args, N, L, stream, tune);
     if (const int S = cluster_form(N, L, args.G, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
         return launch_cluster_s(args, N, L, S, stream, tune);
     if (split_applies(N, L, args.G, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
@@ -817,7 +856,7 @@ __global__ void __launch_bounds__(256) ks_kernel(const uint32_t* __restrict__ a_
                                                  const uint32_t* __restrict__ b_in, const KsKey key,
                                                  int n_big, int n, int l, int log2_beta,
                                                  uint32_t* __restrict__ a_out, uint32_t* __restrict__ b_out,
-                                                 long long B) {
+                                                 long long B, int i_len) {
     __shared__ int dig[KS_TB][KS_KC * KS_LMAX + 1];
     __shared__ __align__(16) uint32_t kt[KS_KC * KS_LMAX][KS_TO];
     const int tid = threadIdx.x;
@@ -832,7 +871,9 @@ __global__ void __launch_bounds__(256) ks_kernel(const uint32_t* __restrict__ a_
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0u;
 
-    for (int i0 = 0; i0 < n_big; i0 += KS_KC) {
+    // blockIdx.z: this block's range of input coefficients (a multiple of KS_KC)
+    const int i_beg = blockIdx.z * i_len, i_end = min(n_big, i_beg + i_len);
+    for (int i0 = i_beg; i0 < i_end; i0 += KS_KC) {
         for (int idx = tid; idx < KS_TB * KS_KC; idx += 256) {
             const int ct = idx / KS_KC, c = idx % KS_KC;
             const long long row = r0 + ct;
@@ -879,7 +920,10 @@ __global__ void __launch_bounds__(256) ks_kernel(const uint32_t* __restrict__ a_
 #pragma unroll
         for (int oo = 0; oo < 4; ++oo) {
             const int o = o0 + tx * 4 + oo;
-            if (o < n) a_out[row * n + o] = acc[cc][oo];
+            if (gridDim.z > 1) {                      // outputs hold 0 and b_in; sums modulo 2^32 commute
+                if (o < n) atomicAdd(a_out + row * n + o, acc[cc][oo]);
+                else if (o == n) atomicAdd(b_out + row, acc[cc][oo]);
+            } else if (o < n) a_out[row * n + o] = acc[cc][oo];
             else if (o == n) b_out[row] = b_in[row] + acc[cc][oo];
         }
     }
@@ -888,9 +932,24 @@ __global__ void __launch_bounds__(256) ks_kernel(const uint32_t* __restrict__ a_
 static int launch_ks_key(const KsKey& key, int n_big, int n, int l, int log2_beta, const uint32_t* a_in,
                          const uint32_t* b_in, uint32_t* a_out, uint32_t* b_out, long long B, cudaStream_t stream) {
     if (B == 0) return TFHE_OK;
-    const dim3 grid((n + 1 + KS_TO - 1) / KS_TO, (unsigned)((B + KS_TB - 1) / KS_TB));
+    // Few ciphertexts give few tiles, each a serial sum over n_big l key rows:
+    // the input coefficients are then split over blockIdx.z, up to about two
+    // blocks per SM and at least four steps each, the parts added by atomics
+    // (32 ciphertexts, 1024 -> 630, 5 levels: 828 -> 60 us)
+    const long long tiles = (long long)((n + 1 + KS_TO - 1) / KS_TO) * ((B + KS_TB - 1) / KS_TB);
+    const long long want = std::max<long long>(1, 2 * std::max(1, sm_count()) / tiles);
+    const int steps = (n_big + KS_KC - 1) / KS_KC;
+    const int per = (int)std::max<long long>(4, (steps + want - 1) / want);
+    const unsigned parts = (unsigned)((steps + per - 1) / per);
+    if (parts > 1) {
+        TFHE_TRY(check_cuda(cudaMemsetAsync(a_out, 0, (size_t)B * n * sizeof(uint32_t), stream), "key switch outputs"));
+        if (b_out != b_in)
+            TFHE_TRY(check_cuda(cudaMemcpyAsync(b_out, b_in, (size_t)B * sizeof(uint32_t), cudaMemcpyDeviceToDevice, stream),
+                                "key switch outputs"));
+    }
+    const dim3 grid((n + 1 + KS_TO - 1) / KS_TO, (unsigned)((B + KS_TB - 1) / KS_TB), parts);
     count_launch();
-    ks_kernel<<<grid, 256, 0, stream>>>(a_in, b_in, key, n_big, n, l, log2_beta, a_out, b_out, B);
+    ks_kernel<<<grid, 256, 0, stream>>>(a_in, b_in, key, n_big, n, l, log2_beta, a_out, b_out, B, per * KS_KC);
     return check_cuda(cudaGetLastError(), "key switch launch");
 }
 
@@ -1108,6 +1167,7 @@ static void keys_free(tfhe_keys* k) {
     cudaFree(k->bsk_mma);
     cudaFree(k->ksk);
     cudaFree(k->ksk_limbs);
+    scratch_trim(k->device);
     delete k;
 }
 
@@ -1119,13 +1179,13 @@ static long long launch_count() { return g_launches.load(std::memory_order_relax
 // parameters that kernel takes
 static int make_mma_key(tfhe_keys* k, cudaStream_t stream) {
     const tfhe_params& p = k->p;
-    if (!mma_form(p.N, p.l_bs, k->M, p.log2_beta_bs, p.log2_q != 32, false, k->ring_kr)) return TFHE_OK;
+    if (k->ring_kr > 0 || !mma_form(p.N, p.l_bs, k->M, p.log2_beta_bs, p.log2_q)) return TFHE_OK;
     const size_t bytes = (size_t)4 * k->G * k->M * p.l_bs * (p.N / 2) * sizeof(double2);
     TFHE_TRY(check_cuda(cudaMalloc(&k->bsk_mma, bytes), "cudaMalloc(bsk, contraction layout)"));
     k->bytes += (int64_t)bytes;
     const BmConvArgs ca{k->bsk, k->bsk_mma, k->G, k->M, p.l_bs};
     count_launch();
-    bm_key_logn10()<<<(unsigned)(std::max(1, sm_count()) * 8), 256, 0, stream>>>(ca);
+    bm_key()<<<(unsigned)(std::max(1, sm_count()) * 8), 256, 0, stream>>>(ca);
     TFHE_TRY(check_cuda(cudaGetLastError(), "bsk layout launch"));
     return check_cuda(cudaStreamSynchronize(stream), "bsk layout");
 }
@@ -1218,7 +1278,28 @@ int tfhe_mul_bootstrap(void* stream, const int64_t* ct_init, int64_t ct_elems, c
     a.indices = indices;
     a.out_i64 = out;
     a.n_lut = 1;
-    return launch_br(a, (int)degree, (int)l, true, 0, static_cast<cudaStream_t>(stream));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // Where the matrix-instruction kernels take the parameters: the caller's key
+    // into their layout (n=630: 165 MB, about 80 us), then the native path's
+    // launches, X^r from the index (n=630, 32 ciphertexts: 6.3 -> 1.3 ms with
+    // the conversion).  The scratch is stream-ordered; where the caller leaves
+    // no memory for it, the key is read in place as below.
+    if (k_override() <= 0 && persistent_launch(nullptr) &&
+        mma_form((int)degree, (int)l, (int)M, (int)log2_beta, (int)log2_q)) {
+        double* key = nullptr;
+        if (scratch_alloc((void**)&key, (size_t)G * 4 * l * M * D * sizeof(double2), st) == cudaSuccess) {
+            const BmRefConvArgs ca{a.bsk, key, (int)M, (int)l};
+            count_launch();
+            bm_ref_key()<<<(unsigned)(G * 2 * l * M), 256, 0, st>>>(ca);
+            int rc = check_cuda(cudaGetLastError(), "bsk layout launch");
+            a.bsk_mma = key;
+            if (rc == TFHE_OK) rc = launch_mma(a, (int)degree, (int)l, st, nullptr);
+            const int rc2 = check_cuda(cudaFreeAsync(key, st), "cudaFreeAsync(bsk layout)");
+            return rc != TFHE_OK ? rc : rc2;
+        }
+        cudaGetLastError();
+    }
+    return launch_br(a, (int)degree, (int)l, true, 0, st);
 }
 
 int tfhe_keys_create(const tfhe_params* params, const uint32_t* bsk_coeff, const uint32_t* ksk_a,
@@ -1448,8 +1529,8 @@ int tfhe_pbs(const tfhe_keys* keys, const uint32_t* a_in, const uint32_t* b_in, 
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const size_t n = (size_t)keys->p.n;
     uint32_t* ks = nullptr;
-    TFHE_TRY(check_cuda(cudaMallocAsync(&ks, (size_t)batch * (n + 1) * sizeof(uint32_t), stream),
-                        "cudaMallocAsync(key-switch output)"));
+    TFHE_TRY(check_cuda(scratch_alloc((void**)&ks, (size_t)batch * (n + 1) * sizeof(uint32_t), stream),
+                        "working memory (key-switch output)"));
     uint32_t* ks_b = ks + (size_t)batch * n;
     int rc = launch_ks(keys, a_in, b_in, ks, ks_b, batch, stream);
     if (rc == TFHE_OK)
@@ -1494,8 +1575,8 @@ int tfhe_pbs_host(const tfhe_keys* keys, const uint32_t* a_host, const uint32_t*
     const size_t slot_words = (size_t)C * nb + C + lut_words + (size_t)C * (n + 1) + (size_t)C * n_lut * N +
                               (size_t)C * n_lut;
     uint32_t* scratch = nullptr;
-    TFHE_TRY(check_cuda(cudaMallocAsync(&scratch, 2 * slot_words * sizeof(uint32_t), stream),
-                        "cudaMallocAsync(host pipeline)"));
+    TFHE_TRY(check_cuda(scratch_alloc((void**)&scratch, 2 * slot_words * sizeof(uint32_t), stream),
+                        "working memory (host pipeline)"));
     struct Slot {
         uint32_t *a, *b, *lut, *ks, *oa, *ob;
     } slot[2];

@@ -713,7 +713,7 @@ static int launch_l2(const KsTcArgs& args, cudaStream_t stream) {
     if (rc != TFHE_OK) return rc;
     int8_t* dig = nullptr;
     if (args.allow_alloc) {
-        rc = check_cuda(cudaMallocAsync((void**)&dig, (size_t)(args.B * K), stream), "cudaMallocAsync(digits)");
+        rc = check_cuda(scratch_alloc((void**)&dig, (size_t)(args.B * K), stream), "working memory (digits)");
         if (rc != TFHE_OK) return rc;
         const long long words = args.B * (long long)args.n_big;
         count_launch();

@@ -94,14 +94,20 @@ BrKernel br_warp32_logn11(int NP);
 BrKernel br_warp64_logn11();
 inline BrKernel br_warp_kernel_for(bool t64, int NP) { return t64 ? br_warp64_logn11() : br_warp32_logn11(NP); }
 
-// the matrix-instruction kernels (four ciphertexts per CTA), N = 1024, l_bs 2
-// or 3, four or eight patterns, and their key layout
+// the matrix-instruction kernels at N = 1024, l_bs 2 or 3, four or eight
+// patterns: four ciphertexts per CTA (C = 1) or per cluster of C = 2, 4 or 8
+// CTAs, on the native buffers or the drop-in's; and their key layout from the
+// native key or the reference's
 using BmConvKernel = void (*)(const BmConvArgs);
-BrKernel br_mma_logn10(int L, int M);
-// the same on clusters of C = 2, 4 or 8 CTAs for four ciphertexts
-BrKernel br_mma_cluster_logn10(int L, int M, int C);
-size_t br_mma_cluster_smem_for(int L, int M, int C);
-BmConvKernel bm_key_logn10();
+using BmRefConvKernel = void (*)(const BmRefConvArgs);
+BrKernel br_mma_native(int L, int M, int C);
+BrKernel br_mma_ref(int L, int M, int C);
+inline BrKernel br_mma_kernel_for(int L, int M, int C, bool ref) {
+    return ref ? br_mma_ref(L, M, C) : br_mma_native(L, M, C);
+}
+size_t br_mma_smem_for(int L, int M, int C);
+BmConvKernel bm_key();
+BmRefConvKernel bm_ref_key();
 
 inline BrConvKernel bsk_fft_kernel_for(int logn) {
     switch (logn) {

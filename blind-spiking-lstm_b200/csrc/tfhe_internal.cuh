@@ -39,6 +39,10 @@ void count_launch();
 // bound of every mbarrier wait, in clock cycles (about 2 s)
 constexpr long long WAIT_LIMIT_CYCLES = 4000000000LL;
 int fail(int code, const std::string& msg);
+// the dynamic shared-memory attribute of a kernel, raised once per device and size
+int smem_attr_once(const void* kern, size_t smem);
+// stream-ordered working memory of one call (freed with cudaFreeAsync)
+cudaError_t scratch_alloc(void** out, size_t bytes, cudaStream_t stream);
 int check_cuda(cudaError_t e, const char* what);
 
 // ----------------------------------------------------------------------------

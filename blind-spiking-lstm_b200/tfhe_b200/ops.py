@@ -48,7 +48,7 @@ def _u32_bits(x: torch.Tensor) -> torch.Tensor:
 
 def all_binary_vectors(m: int, device=None) -> torch.Tensor:
     """cuTFHE/utils.py:5-8: {0,1}^m in meshgrid 'ij' order, (2^m, m) int32."""
-    values = torch.tensor([0, 1], dtype=torch.int32, device=device)
+    values = torch.arange(2, dtype=torch.int32, device=device)       # made on the device: no copy to wait for
     grids = torch.meshgrid(*([values] * m), indexing="ij")
     return torch.stack(grids, dim=-1).reshape(-1, m)
 

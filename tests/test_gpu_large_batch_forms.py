@@ -71,3 +71,34 @@ def test_n1024_matches_one_per_cta(l_bs, log2_beta, collapse):
     small = [1, 3, 4, 5, sms // 4, sms // 2, sms // 2 + 1, sms - 20, sms]
     for i, batch in enumerate(small + _batches()):
         _compare(keys, p, torch.int32, p.n, batch, (1, 4)[i % 2], 100 * collapse + i)
+
+
+@pytest.mark.parametrize("l_bs,log2_beta,collapse", [(3, 7, 3), (2, 8, 2), (3, 9, 3)])
+def test_dropin_n1024_matches_native_words(l_bs, log2_beta, collapse):
+    """multiply_seq_monomial from the reference's key spectra, over every form of
+    the matrix-instruction kernels, against the native one-per-CTA kernel on the
+    same key (base 2^9 keeps the general kernel on both sides)."""
+    from tfhe_b200 import ops
+    p = ParamSet("n66_N1024", N=1024, n=66 if collapse == 3 else 64, log2_beta_bs=log2_beta, l_bs=l_bs,
+                 collapse=collapse, log2_beta_ks=3, l_ks=5, sigma_glwe=2.0 ** 7, sigma_lwe=2.0 ** 17)
+    k = client.keygen(p, 5)
+    keys = Keys.create(p, k.bsk, k.ksk_a, k.ksk_b)
+    j = torch.arange(p.N, device="cuda", dtype=torch.float64)
+    coeff = torch.from_numpy(client._centred(k.bsk)).cuda().to(torch.float64)          # (in, out, G M, l, N)
+    four = torch.fft.fft(coeff * torch.exp(-1j * np.pi * j / p.N))[..., : p.N // 2].permute(1, 0, 3, 2, 4).contiguous()
+    angle = (torch.arange(2 * p.N, device="cuda")[:, None] * (2 * torch.arange(p.N // 2, device="cuda") + 1)) % (2 * p.N)
+    rot = torch.exp(-1j * np.pi * angle.to(torch.float64) / p.N)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    for batch in (1, 4, sms // 4, sms // 2 + 1, sms, 2 * sms, 4 * sms + 1):
+        a = torch.randint(-2 ** 31, 2 ** 31 - 1, (batch, p.n), device="cuda", generator=g, dtype=torch.int32)
+        for shared in (True, False):
+            lut = torch.randint(-2 ** 31, 2 ** 31 - 1, (1 if shared else batch, 2, p.N), device="cuda", generator=g,
+                                dtype=torch.int32)
+            got = ops.multiply_seq_monomial(lut.to(torch.float64), a.to(torch.float64), four, 32, log2_beta, l_bs, p.N,
+                                            collapse, rot, 2)
+            keys.set_tuning(ciphertexts_per_cta=1)
+            want = keys.blind_rotate(a, torch.zeros(batch, dtype=torch.int32, device="cuda"), lut, 2)
+            keys.set_tuning()
+            assert torch.equal((got.to(torch.int64) & 0xFFFFFFFF), (want.to(torch.int64) & 0xFFFFFFFF)), (batch, shared)
