@@ -1,8 +1,8 @@
 // Operators of one encrypted Spike-LSTM timestep around the programmable
 // bootstrap (nn_tfhe/Spike_LSTM.py:15-62, 103-184):
 //
-//   linear_extract_kernel   Linear.__call__: plaintext weight polynomial x
-//                           RLWE, sample_extract at 0, + bias
+//   linear_kernel           Linear.__call__: plaintext weight polynomial x
+//                           RLWE, sample_extract at 0, + bias (lstm_linear.cuh)
 //   lut_mul_sum_kernel      prepare_LUT's multiply_plaintext_ciphertext and
 //                           the sum over the packed sub-LUTs
 //   trace_pack_kernel       pack_lwe_to_rlwe: modulus switch to q/N, trivial
@@ -20,104 +20,11 @@
 #include <string>
 
 #include "tfhe_b200.h"
+#include "lstm_linear.cuh"
 #include "tfhe_dispatch.h"
 #include "tfhe_internal.cuh"
 
 namespace tfhe {
-
-// ---------------------------------------------------------------- linear
-// P_A = W_j(X) A_s(X) mod X^N + 1; the LWE of coefficient 0 is
-// a'[0] = P_A[0], a'[i] = -P_A[N - i] (schemas/text_jax.py:191-208) and
-// b' = P_B[0] + bias_j (Spike_LSTM.py:48-58).
-constexpr int LIN_JT = 4;      // outputs per CTA
-constexpr int LIN_NT = 256;
-
-__global__ void __launch_bounds__(LIN_NT) linear_extract_kernel(const int32_t* __restrict__ W,
-                                                                const int32_t* __restrict__ bias, int J,
-                                                                const uint32_t* __restrict__ ct, int N,
-                                                                uint32_t* __restrict__ out_a,
-                                                                uint32_t* __restrict__ out_b) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint32_t* A = reinterpret_cast<uint32_t*>(smem_raw);            // N
-    int32_t* Ws = reinterpret_cast<int32_t*>(A + N);                // LIN_JT * N
-    __shared__ uint32_t red[LIN_JT][LIN_NT / 32];
-    const int tid = threadIdx.x;
-    const long long s = blockIdx.y;
-    const int j0 = blockIdx.x * LIN_JT;
-    const uint32_t* a_in = ct + s * 2 * N;
-    const uint32_t* b_in = a_in + N;
-    for (int i = tid; i < N; i += LIN_NT) A[i] = a_in[i];
-    for (int i = tid; i < LIN_JT * N; i += LIN_NT) {
-        const int jt = i / N;
-        Ws[i] = (j0 + jt < J) ? W[(long long)(j0 + jt) * N + (i - jt * N)] : 0;
-    }
-    __syncthreads();
-
-    // b' = sum_m W[m] B[-m]: B[0] for m = 0, -B[N - m] otherwise
-    uint32_t pb[LIN_JT];
-#pragma unroll
-    for (int jt = 0; jt < LIN_JT; ++jt) pb[jt] = 0u;
-    for (int m = tid; m < N; m += LIN_NT) {
-        const uint32_t bv = m == 0 ? b_in[0] : 0u - b_in[N - m];
-#pragma unroll
-        for (int jt = 0; jt < LIN_JT; ++jt) pb[jt] += (uint32_t)Ws[jt * N + m] * bv;
-    }
-#pragma unroll
-    for (int jt = 0; jt < LIN_JT; ++jt) {
-        uint32_t v = pb[jt];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((tid & 31) == 0) red[jt][tid >> 5] = v;
-    }
-
-    // every thread owns coefficients c = tid + LIN_NT * r of P_A
-    constexpr int CPT_MAX = 16;                      // N <= 4096
-    uint32_t acc[LIN_JT][CPT_MAX];
-    const int cpt = N / LIN_NT > 0 ? N / LIN_NT : 1;
-#pragma unroll
-    for (int jt = 0; jt < LIN_JT; ++jt)
-#pragma unroll
-        for (int r = 0; r < CPT_MAX; ++r) acc[jt][r] = 0u;
-    for (int m = 0; m < N; ++m) {
-        int32_t w[LIN_JT];
-        bool any = false;
-#pragma unroll
-        for (int jt = 0; jt < LIN_JT; ++jt) {
-            w[jt] = Ws[jt * N + m];
-            any |= w[jt] != 0;
-        }
-        if (!any) continue;                           // uniform across the CTA
-#pragma unroll
-        for (int r = 0; r < CPT_MAX; ++r) {
-            if (r >= cpt) break;
-            const int c = tid + LIN_NT * r;
-            if (c >= N) break;
-            const int idx = c - m;
-            const uint32_t v = idx >= 0 ? A[idx] : 0u - A[idx + N];
-#pragma unroll
-            for (int jt = 0; jt < LIN_JT; ++jt) acc[jt][r] += (uint32_t)w[jt] * v;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int jt = 0; jt < LIN_JT; ++jt) {
-        const int j = j0 + jt;
-        if (j >= J) break;
-        uint32_t* dst = out_a + (s * J + j) * (long long)N;
-#pragma unroll
-        for (int r = 0; r < CPT_MAX; ++r) {
-            if (r >= cpt) break;
-            const int c = tid + LIN_NT * r;
-            if (c >= N) break;
-            if (c == 0) dst[0] = acc[jt][r];
-            else dst[N - c] = 0u - acc[jt][r];
-        }
-        if (tid == 0) {
-            uint32_t v = (uint32_t)bias[j];
-            for (int w = 0; w < LIN_NT / 32; ++w) v += red[jt][w];
-            out_b[s * J + j] = v;
-        }
-    }
-}
 
 // ---------------------------------------------------------------- LUT x RLWE
 // out[s][k] = sum_{g < G} P[g][k](X) * ct[s][g][k] (both polynomials),
@@ -177,16 +84,15 @@ __global__ void __launch_bounds__(LM_NT) lut_mul_sum_kernel(const int32_t* __res
     }
 }
 
-// ---------------------------------------------------------------- trace
-struct TraceArgs {
-    const uint32_t* lwe_a;     // (R, N)
-    const uint32_t* lwe_b;     // (R)
-    const double2* key;        // [step][level][2][H] position order
-    const double2* qt;
-    const double2* tw;
-    int log2_beta, l, steps;
-    uint32_t* out;             // (R, 2, N)
-};
+// The same sums where the LUTs are small (the layer's step LUTs hold 0 / +-1):
+// in the folded FP64 Fourier domain, all groups of one (slot, sequence) in one
+// block.  With G N max|LUT| <= 2^14 a result is below 2^45 and its float64
+// error, at most about 40 2^-53 times that, below 1/4, so it rounds to the
+// exact integer; a block whose LUTs are larger takes the direct sums instead
+// (block-uniform).  A tick of three requests (hidden 256, N = 1024): 1.21 ms
+// with the direct sums.
+constexpr int LF_NT = 256;
+constexpr long long LF_BOUND = 1 << 14;
 
 template <int LOGH, int s>
 __device__ __forceinline__ void forward_all(double2* polys, int npoly, const double2* tw, int tid, int nt) {
@@ -205,6 +111,121 @@ __device__ __forceinline__ void inverse_all(double2* polys, int npoly, const dou
         inverse_all<LOGH, s - 1>(polys, npoly, tw, tid, nt);
     }
 }
+
+// shared memory: two sums and three spectra for each of gc groups at a time
+inline size_t lut_fft_smem(int N, int gc) { return (size_t)(2 + 3 * gc) * (N / 2) * sizeof(double2); }
+
+template <int LOGN>
+__global__ void __launch_bounds__(LF_NT) lut_fft_kernel(const int32_t* __restrict__ P, int G, int Kp,
+                                                        const uint32_t* __restrict__ ct, const double2* qt,
+                                                        const double2* tw, int gc, uint32_t* __restrict__ out) {
+    constexpr int N = 1 << LOGN, H = N / 2, LOGH = LOGN - 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* sum = reinterpret_cast<double2*>(smem_raw);        // 2 H
+    double2* work = sum + 2 * H;                                // 3 gc H: (LUT, mask, body) of each group
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int k = blockIdx.x;
+    const long long s = blockIdx.y;
+    uint32_t* dst = out + (s * Kp + k) * 2 * (long long)N;
+
+    uint32_t most = 0u;
+    for (int g = 0; g < G; ++g)
+        for (int i = tid; i < N; i += nt) {
+            const int v = P[((long long)g * Kp + k) * N + i];
+            most = max(most, v < 0 ? 0u - (uint32_t)v : (uint32_t)v);
+        }
+    if (__syncthreads_or((long long)most * G * N > LF_BOUND)) {
+        // direct negacyclic sums (lut_mul_sum_kernel's operations)
+        uint32_t* A = reinterpret_cast<uint32_t*>(smem_raw);
+        uint32_t* B = A + N;
+        int32_t* Ps = reinterpret_cast<int32_t*>(B + N);
+        constexpr int CPT = N / LF_NT > 0 ? N / LF_NT : 1;
+        uint32_t acc_a[CPT], acc_b[CPT];
+#pragma unroll
+        for (int r = 0; r < CPT; ++r) acc_a[r] = acc_b[r] = 0u;
+        for (int g = 0; g < G; ++g) {
+            const uint32_t* src = ct + ((s * G + g) * (long long)Kp + k) * 2 * N;
+            const int32_t* lut = P + ((long long)g * Kp + k) * N;
+            for (int i = tid; i < N; i += nt) {
+                A[i] = src[i];
+                B[i] = src[N + i];
+                Ps[i] = lut[i];
+            }
+            __syncthreads();
+            for (int m = 0; m < N; ++m) {
+                const int32_t w = Ps[m];
+                if (w == 0) continue;
+#pragma unroll
+                for (int r = 0; r < CPT; ++r) {
+                    const int c = tid + LF_NT * r;
+                    if (c >= N) break;
+                    const int idx = c - m;
+                    acc_a[r] += (uint32_t)w * (idx >= 0 ? A[idx] : 0u - A[idx + N]);
+                    acc_b[r] += (uint32_t)w * (idx >= 0 ? B[idx] : 0u - B[idx + N]);
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int r = 0; r < CPT; ++r) {
+            const int c = tid + LF_NT * r;
+            if (c >= N) break;
+            dst[c] = acc_a[r];
+            dst[N + c] = acc_b[r];
+        }
+        return;
+    }
+
+    for (int g0 = 0; g0 < G; g0 += gc) {
+        const int ng = min(gc, G - g0);
+        for (int x = tid; x < ng * H; x += nt) {
+            const int g = x / H, i = x % H;
+            const int32_t* lut = P + ((long long)(g0 + g) * Kp + k) * N;
+            const uint32_t* src = ct + ((s * G + g0 + g) * (long long)Kp + k) * 2 * N;
+            const double2 w = qt[i];
+            auto fold = [&](int which, double lo, double hi) {
+                work[(size_t)(3 * g + which) * H + swz(i)] =
+                    make_double2(fma(w.x, lo, w.y * hi), fma(w.y, lo, -w.x * hi));
+            };
+            fold(0, (double)lut[i], (double)lut[i + H]);
+            fold(1, (double)(int32_t)src[i], (double)(int32_t)src[i + H]);
+            fold(2, (double)(int32_t)src[N + i], (double)(int32_t)src[N + i + H]);
+        }
+        __syncthreads();
+        forward_all<LOGH, 0>(work, 3 * ng, tw, tid, nt);
+        for (int p = tid; p < H; p += nt) {
+            const int e = swz(p);
+            double2 sa = g0 ? sum[e] : make_double2(0.0, 0.0), sb = g0 ? sum[H + e] : make_double2(0.0, 0.0);
+            for (int g = 0; g < ng; ++g) {
+                const double2 f = work[(size_t)(3 * g) * H + e];
+                c_mac(sa, f, work[(size_t)(3 * g + 1) * H + e]);
+                c_mac(sb, f, work[(size_t)(3 * g + 2) * H + e]);
+            }
+            sum[e] = sa;
+            sum[H + e] = sb;
+        }
+        __syncthreads();
+    }
+    inverse_all<LOGH, Plan<LOGH>::NS - 1>(sum, 2, tw, tid, nt);
+    constexpr double inv_h = 1.0 / H;
+    for (int x = tid; x < 2 * H; x += nt) {
+        const int a = x / H, i = x % H;
+        const double2 u = c_mul(c_conj(qt[i]), sum[(size_t)a * H + swz(i)]);
+        dst[a * N + i] = (uint32_t)__double2ll_rn(u.x * inv_h);
+        dst[a * N + i + H] = (uint32_t)__double2ll_rn(-u.y * inv_h);
+    }
+}
+
+// ---------------------------------------------------------------- trace
+struct TraceArgs {
+    const uint32_t* lwe_a;     // (R, N)
+    const uint32_t* lwe_b;     // (R)
+    const double2* key;        // [step][level][2][H] position order
+    const double2* qt;
+    const double2* tw;
+    int log2_beta, l, steps;
+    uint32_t* out;             // (R, 2, N)
+};
 
 __device__ __forceinline__ double cmod_q32(double x) {
     const double q = 4294967296.0;
@@ -549,12 +570,7 @@ int tfhe_linear_extract(const int32_t* weights, const int32_t* bias, int32_t J, 
     if (!weights || !bias || !rlwe || !out_a || !out_b)
         return fail(TFHE_ERR_INVALID_ARGUMENT, "linear: null pointer");
     if (S > 65535) return fail(TFHE_ERR_INVALID_ARGUMENT, "linear: at most 65535 ciphertexts per call");
-    const size_t smem = (size_t)N * sizeof(uint32_t) + (size_t)LIN_JT * N * sizeof(int32_t);
-    TFHE_TRY(smem_attr_once((const void*)linear_extract_kernel, smem));
-    const dim3 grid((J + LIN_JT - 1) / LIN_JT, (unsigned)S);
-    count_launch();
-    linear_extract_kernel<<<grid, LIN_NT, smem, (cudaStream_t)stream>>>(weights, bias, J, rlwe, N, out_a, out_b);
-    return check_cuda(cudaGetLastError(), "linear kernel launch");
+    return launch_linear<uint32_t, int32_t>(weights, bias, J, rlwe, S, N, out_a, out_b, (cudaStream_t)stream);
 }
 
 int tfhe_lut_mul_sum(const int32_t* luts, int32_t groups, int32_t per_group, const uint32_t* rlwe, int64_t S,
@@ -564,9 +580,27 @@ int tfhe_lut_mul_sum(const int32_t* luts, int32_t groups, int32_t per_group, con
     if (per_group == 0 || S == 0) return TFHE_OK;
     if (!luts || !rlwe || !out) return fail(TFHE_ERR_INVALID_ARGUMENT, "lut product: null pointer");
     if (S > 65535) return fail(TFHE_ERR_INVALID_ARGUMENT, "lut product: at most 65535 sequences per call");
+    const dim3 grid((unsigned)per_group, (unsigned)S);
+    if (N <= 2048) {
+        const FftPlan* pl = get_plan(N);
+        if (!pl) return TFHE_ERR_INTERNAL;
+        // groups at a time: all that fit in 112 KB, so two blocks share an SM
+        const int gc = std::min<int>(groups, std::max<int>(1, (int)((112 * 1024 / (N / 2 * sizeof(double2)) - 2) / 3)));
+        const size_t smem = lut_fft_smem(N, gc);
+        int logn = 7;
+        while ((1 << logn) < N) ++logn;
+        auto kern = logn == 7   ? lut_fft_kernel<7>
+                    : logn == 8  ? lut_fft_kernel<8>
+                    : logn == 9  ? lut_fft_kernel<9>
+                    : logn == 10 ? lut_fft_kernel<10>
+                                 : lut_fft_kernel<11>;
+        TFHE_TRY(smem_attr_once((const void*)kern, smem));
+        count_launch();
+        kern<<<grid, LF_NT, smem, (cudaStream_t)stream>>>(luts, groups, per_group, rlwe, pl->qt, pl->tw, gc, out);
+        return check_cuda(cudaGetLastError(), "lut product launch");
+    }
     const size_t smem = 3 * (size_t)N * sizeof(uint32_t);
     TFHE_TRY(smem_attr_once((const void*)lut_mul_sum_kernel, smem));
-    const dim3 grid((unsigned)per_group, (unsigned)S);
     count_launch();
     lut_mul_sum_kernel<<<grid, LM_NT, smem, (cudaStream_t)stream>>>(luts, groups, per_group, rlwe, N, out);
     return check_cuda(cudaGetLastError(), "lut product launch");

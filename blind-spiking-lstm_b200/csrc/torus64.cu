@@ -8,7 +8,8 @@
 //                           (cuTFHE/multiply.py:67-79) from 64-bit masks
 //   rotate_extract64_kernel rotation by -b~ and many-LUT sample extraction
 //                           (schemas/RLWE_jax.py:295-303)
-//   linear64_kernel         Linear.__call__ (nn_tfhe/Spike_LSTM.py:48-58)
+//   linear_kernel           Linear.__call__ (nn_tfhe/Spike_LSTM.py:48-58;
+//                           lstm_linear.cuh)
 //   lut_mul_sum64_kernel    prepare_LUT's product summed over the packed
 //                           sub-LUTs (nn_tfhe/activation.py:103-106,
 //                           nn_tfhe/Spike_LSTM.py:129-132)
@@ -31,6 +32,7 @@
 #include <string>
 
 #include "tfhe_b200.h"
+#include "lstm_linear.cuh"
 #include "tfhe_dispatch.h"
 #include "tfhe_internal.cuh"
 
@@ -184,89 +186,7 @@ __global__ void rotate_extract64_kernel(const long long* __restrict__ acc, const
     }
 }
 
-// ---------------------------------------------------------------- linear
-constexpr int LIN_JT = 4, LIN_NT = 256, CPT_MAX = 16;
-
-__global__ void __launch_bounds__(LIN_NT) linear64_kernel(const int32_t* __restrict__ W,
-                                                          const long long* __restrict__ bias, int J,
-                                                          const u64* __restrict__ ct, int N, u64* __restrict__ out_a,
-                                                          u64* __restrict__ out_b) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    u64* A = reinterpret_cast<u64*>(smem_raw);                   // N
-    int32_t* Ws = reinterpret_cast<int32_t*>(A + N);             // LIN_JT * N
-    __shared__ u64 red[LIN_JT][LIN_NT / 32];
-    const int tid = threadIdx.x;
-    const long long s = blockIdx.y;
-    const int j0 = blockIdx.x * LIN_JT;
-    const u64* a_in = ct + s * 2 * N;
-    const u64* b_in = a_in + N;
-    for (int i = tid; i < N; i += LIN_NT) A[i] = a_in[i];
-    for (int i = tid; i < LIN_JT * N; i += LIN_NT) {
-        const int jt = i / N;
-        Ws[i] = (j0 + jt < J) ? W[(long long)(j0 + jt) * N + (i - jt * N)] : 0;
-    }
-    __syncthreads();
-    u64 pb[LIN_JT];
-#pragma unroll
-    for (int jt = 0; jt < LIN_JT; ++jt) pb[jt] = 0ULL;
-    for (int m = tid; m < N; m += LIN_NT) {
-        const u64 bv = m == 0 ? b_in[0] : 0ULL - b_in[N - m];
-#pragma unroll
-        for (int jt = 0; jt < LIN_JT; ++jt) pb[jt] += (u64)(long long)Ws[jt * N + m] * bv;
-    }
-#pragma unroll
-    for (int jt = 0; jt < LIN_JT; ++jt) {
-        u64 v = pb[jt];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((tid & 31) == 0) red[jt][tid >> 5] = v;
-    }
-    u64 acc[LIN_JT][CPT_MAX];
-    const int cpt = N / LIN_NT > 0 ? N / LIN_NT : 1;
-#pragma unroll
-    for (int jt = 0; jt < LIN_JT; ++jt)
-#pragma unroll
-        for (int r = 0; r < CPT_MAX; ++r) acc[jt][r] = 0ULL;
-    for (int m = 0; m < N; ++m) {
-        int32_t w[LIN_JT];
-        bool any = false;
-#pragma unroll
-        for (int jt = 0; jt < LIN_JT; ++jt) {
-            w[jt] = Ws[jt * N + m];
-            any |= w[jt] != 0;
-        }
-        if (!any) continue;                           // uniform across the CTA
-#pragma unroll
-        for (int r = 0; r < CPT_MAX; ++r) {
-            if (r >= cpt) break;
-            const int c = tid + LIN_NT * r;
-            if (c >= N) break;
-            const int idx = c - m;
-            const u64 v = idx >= 0 ? A[idx] : 0ULL - A[idx + N];
-#pragma unroll
-            for (int jt = 0; jt < LIN_JT; ++jt) acc[jt][r] += (u64)(long long)w[jt] * v;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int jt = 0; jt < LIN_JT; ++jt) {
-        const int j = j0 + jt;
-        if (j >= J) break;
-        u64* dst = out_a + (s * J + j) * (long long)N;
-#pragma unroll
-        for (int r = 0; r < CPT_MAX; ++r) {
-            if (r >= cpt) break;
-            const int c = tid + LIN_NT * r;
-            if (c >= N) break;
-            if (c == 0) dst[0] = acc[jt][r];
-            else dst[N - c] = 0ULL - acc[jt][r];
-        }
-        if (tid == 0) {
-            u64 v = (u64)bias[j];
-            for (int w = 0; w < LIN_NT / 32; ++w) v += red[jt][w];
-            out_b[s * J + j] = v;
-        }
-    }
-}
+constexpr int CPT_MAX = 16;   // coefficients per thread, N = 4096
 
 // ---------------------------------------------------------------- LUT x RLWE
 constexpr int LM_NT = 256;
@@ -1039,14 +959,9 @@ int tfhe64_linear_extract(const int32_t* weights, const int64_t* bias, int32_t J
     if (J == 0 || S == 0) return TFHE_OK;
     if (!weights || !bias || !rlwe || !out_a || !out_b) return fail(TFHE_ERR_INVALID_ARGUMENT, "linear64: null pointer");
     if (S > 65535) return fail(TFHE_ERR_INVALID_ARGUMENT, "linear64: at most 65535 ciphertexts per call");
-    const size_t smem = (size_t)N * sizeof(u64) + (size_t)LIN_JT * N * sizeof(int32_t);
-    TFHE_TRY(smem_attr_once((const void*)linear64_kernel, smem));
-    const dim3 grid((J + LIN_JT - 1) / LIN_JT, (unsigned)S);
-    count_launch();
-    linear64_kernel<<<grid, LIN_NT, smem, (cudaStream_t)stream>>>(
-        weights, reinterpret_cast<const long long*>(bias), J, reinterpret_cast<const u64*>(rlwe), N,
-        reinterpret_cast<u64*>(out_a), reinterpret_cast<u64*>(out_b));
-    return check_cuda(cudaGetLastError(), "linear64 launch");
+    return launch_linear<u64, long long>(weights, reinterpret_cast<const long long*>(bias), J,
+                                         reinterpret_cast<const u64*>(rlwe), S, N, reinterpret_cast<u64*>(out_a),
+                                         reinterpret_cast<u64*>(out_b), (cudaStream_t)stream);
 }
 
 // LUT products in the Fourier domain (TFHE_B200_LUT_FFT=0: the direct sums)
