@@ -121,6 +121,14 @@ inline BrConvKernel bsk_fft_kernel_for(int logn) {
     }
 }
 
+// the 64-bit trace at N = 2048 (trace_tree.cu): whether keys take it, their
+// layout's complex words
+bool trace_tree_takes(int N, int l, int log2_beta);
+size_t trace_tree_key_words(int l, int steps);
+int trace_tree_key(const unsigned long long* keys, int l, int steps, const FftPlan* pl, double2* dst, cudaStream_t stream);
+int launch_trace_tree(const unsigned long long* lwe_a, const unsigned long long* lwe_b, const double2* key, int l, int log2_beta, int steps, long long R,
+                      unsigned long long* out, const FftPlan* pl, cudaStream_t stream);
+
 // tensor-core LWE key switch (ks_tc.cu)
 struct KsTcArgs {
     const uint32_t* a_in;         // (B, n_big)

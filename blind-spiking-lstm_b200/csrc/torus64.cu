@@ -896,7 +896,8 @@ using namespace tfhe::t64;
 
 struct tfhe64_galois_keys {
     int N = 0, log2_beta = 0, l = 0, steps = 0, device = 0;
-    double2* key = nullptr;     // [steps][l][2][LIMBS][H]
+    double2* key = nullptr;     // [steps][l][2][LIMBS][H], or trace_tree_kernel's layout
+    bool tree = false;
 };
 
 extern "C" {
@@ -1038,9 +1039,12 @@ int tfhe64_galois_keys_create(int32_t N, int32_t log2_beta, int32_t l, const uin
     cudaGetDevice(&gk->device);
     const long long npoly = (long long)gk->steps * l * 2;
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = check_cuda(cudaMalloc(&gk->key, (size_t)npoly * LIMBS * (N / 2) * sizeof(double2)),
-                        "cudaMalloc(galois key64)");
-    if (rc == TFHE_OK) {
+    gk->tree = trace_tree_takes(N, l, log2_beta);
+    const size_t words = gk->tree ? trace_tree_key_words(l, gk->steps) : (size_t)npoly * LIMBS * (N / 2);
+    int rc = check_cuda(cudaMalloc(&gk->key, words * sizeof(double2)), "cudaMalloc(galois key64)");
+    if (rc == TFHE_OK && gk->tree) {
+        rc = trace_tree_key(reinterpret_cast<const u64*>(keys), l, gk->steps, pl, gk->key, st);
+    } else if (rc == TFHE_OK) {
         const u64* src = reinterpret_cast<const u64*>(keys);
 #define T64_LIMB_FFT(LG) launch_limb_fft<LG>(src, npoly, pl, gk->key, st)
         rc = [&]() -> int { T64_DISPATCH(log2_exact(N), T64_LIMB_FFT) }();
@@ -1072,6 +1076,9 @@ int tfhe64_pack_lwe_to_rlwe(const tfhe64_galois_keys* gk, const uint64_t* lwe_a,
     if (R > 2147483647LL) return fail(TFHE_ERR_INVALID_ARGUMENT, "pack_lwe_to_rlwe64: too many ciphertexts");
     const FftPlan* pl = get_plan(gk->N);
     if (!pl) return TFHE_ERR_INTERNAL;
+    if (gk->tree)
+        return launch_trace_tree(reinterpret_cast<const u64*>(lwe_a), reinterpret_cast<const u64*>(lwe_b), gk->key, gk->l,
+                                 gk->log2_beta, gk->steps, R, reinterpret_cast<u64*>(out), pl, (cudaStream_t)stream);
     Trace64Args a{reinterpret_cast<const u64*>(lwe_a), reinterpret_cast<const u64*>(lwe_b), gk->key, pl->qt, pl->tw,
                   gk->log2_beta, gk->l, gk->steps, reinterpret_cast<u64*>(out)};
     cudaStream_t st = (cudaStream_t)stream;

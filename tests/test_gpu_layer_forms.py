@@ -65,3 +65,28 @@ def test_lut_products_exact(N, G, most):
                 for g in range(G):
                     want += _negacyclic(lut[g, k], x[s, g, k, a])
                 assert np.array_equal(got[s, k, a], want), (s, k, a)
+
+
+@pytest.mark.parametrize("log2_beta,l", [(8, 5), (7, 6), (9, 4)])
+def test_trace64_n2048_matches_general_kernel(monkeypatch, log2_beta, l):
+    """The kernel of three limbs against the general one on the same keys, from
+    one LWE to more than a round of CTAs; masks and bodies include zero, the
+    most negative word, and multiples of a digit's half (ties)."""
+    from tfhe_b200 import torus64
+    N = 2048
+    rng = np.random.default_rng(100 * l + log2_beta)
+    keys = _words(rng, (11, l, 2, N), 64)
+    keys[:, 0] = np.uint64(2 ** 64 - 2 ** 63 - 2 ** 42 - 2 ** 21)      # every limb at its largest
+    here = torus64.GaloisKeys64(keys, log2_beta, l)
+    monkeypatch.setenv("TFHE_B200_TRACE_TREE", "0")
+    general = torus64.GaloisKeys64(keys, log2_beta, l)
+    for R in (1, 3, 300):
+        a, b = _words(rng, (R, N), 64), _words(rng, (R,), 64)
+        a[0] = 0
+        if R > 2:
+            a[1] = 1 << 63
+            a[2] <<= 63 - l * log2_beta + 11
+            b[1] = 1 << 63
+            a[-1] = a[-1, 0]                                           # digits that add up
+        got = here.pack_lwe_to_rlwe(_dev(a, 64), _dev(b, 64))
+        assert torch.equal(got, general.pack_lwe_to_rlwe(_dev(a, 64), _dev(b, 64))), R
