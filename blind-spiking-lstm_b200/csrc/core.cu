@@ -954,13 +954,13 @@ static int launch_ks_key(const KsKey& key, int n_big, int n, int l, int log2_bet
 }
 
 static int launch_ks(const tfhe_keys* k, const uint32_t* a_in, const uint32_t* b_in, uint32_t* a_out,
-                     uint32_t* b_out, long long B, cudaStream_t stream) {
+                     uint32_t* b_out, long long B, cudaStream_t stream, bool allow_alloc = true) {
     // the tensor-core kernel reads the input rows with 16-byte loads
     if (k->ksk_limbs && k->tune.ks_tensor_cores != 0 && (reinterpret_cast<uintptr_t>(a_in) & 15) == 0) {
         int* status = device_status_word();
         if (!status) return fail(TFHE_ERR_INTERNAL, "device status word unavailable");
         KsTcArgs args{a_in, b_in, k->ksk_limbs, k->p.n_big, k->p.n, k->p.l_ks, k->p.log2_beta_ks, k->ks_npad, B,
-                      a_out, b_out, WAIT_LIMIT_CYCLES, status, 0, 0, nullptr};
+                      a_out, b_out, WAIT_LIMIT_CYCLES, status, 0, 0, nullptr, false, allow_alloc};
         return launch_ks_tc(args, stream);
     }
     const long long ldk = k->ldk, l = k->p.l_ks;
@@ -1817,7 +1817,7 @@ int tfhe_pbs_noalloc(const tfhe_keys* keys, const uint32_t* a_in, const uint32_t
     uint32_t* ks = nullptr;
     TFHE_TRY(noalloc_base(&ks));
     uint32_t* ks_b = ks + (size_t)batch * n;
-    TFHE_TRY(launch_ks(keys, a_in, b_in, ks, ks_b, batch, stream));
+    TFHE_TRY(launch_ks(keys, a_in, b_in, ks, ks_b, batch, stream, false));
     return br_native(keys, ks, ks_b, lut, lut_count, n_lut, nullptr, out_a, out_b, batch, stream, nullptr);
 }
 

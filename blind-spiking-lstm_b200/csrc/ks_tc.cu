@@ -26,6 +26,7 @@
 #include <cstring>
 #include <mutex>
 #include <set>
+#include <type_traits>
 #include <utility>
 
 #include "tfhe_b200.h"
@@ -296,17 +297,15 @@ __global__ void __launch_bounds__(KTC_THREADS, 1) ks_tc_kernel(KsTcArgs a) {
 // ============================================================================
 // Pipelined form: operands fed by the Tensor Memory Accelerator.
 //
-// The limb key tile (B) of every stage arrives by 2D TMA copies (one 32-byte
-// K slice x 256 limb rows per copy with 32-byte swizzling, or one 16-byte
-// chunk unswizzled; each CTA fetches its own tiles, through a tensor map over
-// this GPU's memory only) into a ring of stages; the digits (A) either arrive the
-// same way from a digit matrix made once per call (tc_digits_kernel) or are
-// computed by 8 producer warps into the ring.  One thread issues the copies,
-// one thread the MMAs; full / empty mbarriers per stage pass the ring between
-// them, so loads of stage s + 1 .. s + S - 1 overlap the MMAs of stage s.
-// Shared layout per stage and operand: with swizzling, [slice][row][32 B]
-// (one 32-byte K slice of all rows, 8-row atoms of 256 bytes, the descriptor's
-// 32-byte swizzle mode); without, and for digits the producers write,
+// The form of calls that may not allocate (and of those that find no memory):
+// the limb key tile (B) of every stage arrives by 2D TMA copies (one 32-byte K
+// slice x 256 limb rows per copy with 32-byte swizzling; each CTA fetches its
+// own tiles, through a tensor map over this GPU's memory only) into a ring of
+// stages; the digits (A) are computed by 8 producer warps into the ring.  One
+// thread issues the copies, one thread the MMAs; full / empty mbarriers per
+// stage pass the ring between them, so loads of stage s + 1 .. s + S - 1
+// overlap the MMAs of stage s.  Shared layout per stage: B [slice][row][32 B]
+// (8-row atoms of 256 bytes, the descriptor's 32-byte swizzle mode); A
 // [chunk][row][16 B], the K-major no-swizzle canonical layout with leading
 // byte offset rows * 16 and stride byte offset 128.
 // ============================================================================
@@ -330,45 +329,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
             "r"(smem_addr(dst)),
         "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar))
         : "memory");
-}
-
-// the gadget digits of one input word, as the one-stage kernel computes them
-template <int L, bool W64>
-__device__ __forceinline__ void word_digits(const void* a_in, long long idx, int log2_beta, int8_t* out) {
-    if constexpr (W64) {
-        long long x = (long long)reinterpret_cast<const unsigned long long*>(a_in)[idx];
-#pragma unroll
-        for (int j = 0; j < L; ++j) {
-            long long rem;
-            out[j] = (int8_t)rne_shift64(x, 64 - (j + 1) * log2_beta, &rem);
-            x = rem;
-        }
-    } else {
-        double x = (double)(int32_t)reinterpret_cast<const uint32_t*>(a_in)[idx] * ldexp(1.0, -32);
-        const double beta = ldexp(1.0, log2_beta);
-#pragma unroll
-        for (int j = 0; j < L; ++j) {
-            const double y = x * beta;
-            const double d = rint(y);
-            x = y - d;
-            out[j] = (int8_t)(int)d;
-        }
-    }
-}
-
-// digit matrix (B, n_big l) int8, row-major: column i l + j = digit j of
-// a_in[row][i] (the A operand of the pipelined kernel)
-template <int L, bool W64>
-__global__ void __launch_bounds__(256) tc_digits_kernel(const void* a_in, long long B, int n_big, int log2_beta,
-                                                        int8_t* __restrict__ out) {
-    const long long total = B * (long long)n_big;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
-        int8_t d[L];
-        word_digits<L, W64>(a_in, idx, log2_beta, d);
-#pragma unroll
-        for (int j = 0; j < L; ++j) out[idx * L + j] = d[j];
-    }
 }
 
 // 16 consecutive input words of one row -> their 16 L digits (the A staging
@@ -468,12 +428,226 @@ __device__ __forceinline__ void store_cols(const KsTcArgs& a, long long row, int
     }
 }
 
-// SW: TMA copies of 32-byte K slices with 32-byte swizzling (one copy per
-// MMA K step, whole 32-byte sectors) instead of 16-byte chunks
-template <int L, bool PACK, bool W64, bool A_TMA, bool SW>
+// store_cols' outputs for one row, 32 accumulator columns at a time: the row's
+// place (a 64-bit division for packing) is found once
+template <bool PACK, bool W64>
+struct ColStore {
+    using word = typename std::conditional<W64, unsigned long long, uint32_t>::type;
+    static constexpr int LIMBS = W64 ? 8 : 4;
+    const KsTcArgs& a;
+    long long row;
+    int t = 0;
+    word* dst = nullptr;                                // packing: the row's RLWE
+    __device__ __forceinline__ ColStore(const KsTcArgs& args, long long r) : a(args), row(r) {
+        if constexpr (PACK) {
+            const long long sq = row / a.pack_T;
+            t = (int)(row - sq * a.pack_T);
+            dst = reinterpret_cast<word*>(a.pack_out) + sq * 2 * (long long)a.pack_N;
+        }
+    }
+    __device__ __forceinline__ void store(int colabs, const uint32_t (&v)[32]) const {
+#pragma unroll
+        for (int h = 0; h < 32 / LIMBS; ++h) {
+            const int o = colabs / LIMBS + h;
+            word val = 0;
+#pragma unroll
+            for (int i = 0; i < LIMBS; ++i) {
+                if constexpr (W64) val += (word)(long long)(int32_t)v[LIMBS * h + i] << (8 * i);
+                else val += v[LIMBS * h + i] << (8 * i);
+            }
+            if constexpr (PACK) {
+                if (o >= 2 * a.pack_N) continue;
+                const int poly = o >= a.pack_N;
+                int d = o - poly * a.pack_N + t;
+                word add = word(0) - val;
+                if (d >= a.pack_N) {
+                    d -= a.pack_N;
+                    add = val;
+                }
+                atomicAdd(dst + poly * a.pack_N + d, add);
+            } else {
+                word* const a_out = reinterpret_cast<word*>(a.a_out) + row * a.n;
+                word* const b_out = reinterpret_cast<word*>(a.b_out) + row;
+                if (gridDim.z > 1) {                    // outputs hold 0 and b_in
+                    if (o <= a.n) atomicAdd(o < a.n ? a_out + o : b_out, val);
+                } else if (o < a.n) a_out[o] = val;
+                else if (o == a.n) *b_out = reinterpret_cast<const word*>(a.b_in)[row] + val;
+            }
+        }
+    }
+};
+
+// digit matrix (rows, n_big l) int8, row-major: column i l + j = digit j of
+// a_in[row][i]; 16 words of a row per thread (a_in 16-byte aligned, n_big % 32 == 0)
+template <int L, bool W64>
+__global__ void __launch_bounds__(256) tc_digits16_kernel(const void* a_in, long long words, int log2_beta,
+                                                          int8_t* __restrict__ out) {
+    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < words / 16;
+         idx += (long long)gridDim.x * blockDim.x) {
+        int8_t d[16 * L];
+        digits16<L, W64>(a_in, idx * 16, log2_beta, d);
+#pragma unroll
+        for (int c = 0; c < L; ++c) {
+            uint4 v;
+            memcpy(&v, d + c * 16, 16);
+            reinterpret_cast<uint4*>(out)[idx * L + c] = v;
+        }
+    }
+}
+
+// ============================================================================
+// Both operands by TMA in 128-byte K blocks: the form of every call that may
+// allocate the digit matrix.
+//
+// With 32-byte K slices (the form above, once fed the digit matrix the same
+// way) packing 2048 LWEs on the 64-bit torus took 1044 us, 1.3 int8 POP/s: TMA
+// works row by row, and 16-byte chunks had taken twice that again.  A copy here
+// brings rows of 128 bytes (128-byte swizzling, four MMA K steps) into a ring of
+// 48 KB slots: 486 us.  What is left is L2 traffic, (rows + columns) per tile
+// and digit; 256 x 256 tiles (two accumulators, all of TMEM, three 64 KB
+// slots) read a third less: 431 us, 3.2 POP/s, the measured bf16 rate twice.
+// The epilogue finds a row's place once, not a 64-bit division per output.
+//
+// Few tiles leave SMs idle, each one a serial sum over all digits: grid.z parts
+// of the K blocks are then added by atomics (sums modulo 2^32 and 2^64
+// commute; packing adds that way anyhow).  Key switch of n=742 (K = 10240), with
+// digits computed inside the kernel before: 256 ciphertexts 157 -> 40 us, 1024
+// 158 -> 52, 16384 1767 -> 457.
+// ============================================================================
+constexpr int KT3_THREADS = 256;
+constexpr int KT3_K = 128;                             // digits per ring slot
+
+constexpr uint32_t kt3_slot_bytes(int tm) { return (uint32_t)(tm * KTC_M + KTC_N) * KT3_K; }
+constexpr size_t kt3_smem(int tm, int slots) { return (size_t)slots * kt3_slot_bytes(tm) + 1024; }
+
+// K-major descriptor of a tile written by TMA with 128-byte swizzling: rows of
+// 128 bytes, 8-row atoms 1024 bytes apart; a 32-byte K step moves the start
+// address inside the atom
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
+    const uint32_t lo = ((saddr >> 4) & 0x3FFFu) | (1u << 16);
+    const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+    return ((uint64_t)hi << 32) | lo;
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+
+template <int TM, int S, bool PACK, bool W64>
+__global__ void __launch_bounds__(KT3_THREADS, 1)
+    ks_tc3_kernel(const KsTcArgs a, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                  int rows_fast, long long first_row, long long rows, int part_steps) {
+    constexpr uint32_t A_BYTES = TM * KTC_M * KT3_K, SLOT = kt3_slot_bytes(TM);
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* smem = smem_dyn + ((1024u - (smem_addr(smem_dyn) & 1023u)) & 1023u);
+    __shared__ __align__(8) uint64_t full[S];
+    __shared__ __align__(8) uint64_t empty[S];
+    __shared__ __align__(8) uint64_t done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int fail;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const long long row0 = (long long)(rows_fast ? blockIdx.x : blockIdx.y) * (TM * KTC_M);
+    const int col0 = (int)(rows_fast ? blockIdx.y : blockIdx.x) * KTC_N;
+    // this part's K blocks (the host leaves none empty; past K both operands read as zero)
+    const int step0 = (int)blockIdx.z * part_steps;
+    const int steps = min(part_steps, (a.n_big * a.l + KT3_K - 1) / KT3_K - step0);
+    volatile int* vfail = &fail;
+    const long long wlim = a.wait_limit < 200000000LL ? a.wait_limit : 200000000LL;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
+                     "r"((uint32_t)(TM * KTC_N)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    if (tid == 0) {
+        for (int i = 0; i < S; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        mbar_init(&done, 1);
+        fail = 0;
+        mbar_fence_init();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == 0 && lane == 0) {
+        int issued = 0;
+        for (int s = 0; s < steps && !*vfail; ++s) {
+            const int slot = s % S;
+            if (s >= S && !mbar_wait_bounded(&empty[slot], (uint32_t)(((s / S) + 1) & 1), wlim, a.status)) {
+                *vfail = 1;
+                break;
+            }
+            unsigned char* st = smem + (size_t)slot * SLOT;
+            mbar_arrive_expect_tx(&full[slot], SLOT);
+            tma_load_2d(st + A_BYTES, &tmB, (step0 + s) * KT3_K, col0, &full[slot]);
+            tma_load_2d(st, &tmA, (step0 + s) * KT3_K, (int)row0, &full[slot]);
+            issued = s + 1;
+        }
+        // this thread's copies still in flight land before the CTA ends
+        for (int s = issued > S ? issued - S : 0; s < issued; ++s)
+            if (!mbar_wait_bounded(&full[s % S], (uint32_t)((s / S) & 1), wlim, a.status)) *vfail = 1;
+    } else if (warp == 1 && lane == 0) {
+        for (int s = 0; s < steps && !*vfail; ++s) {
+            const int slot = s % S;
+            if (!mbar_wait_bounded(&full[slot], (uint32_t)((s / S) & 1), wlim, a.status)) {
+                *vfail = 1;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t sa = smem_addr(smem + (size_t)slot * SLOT);
+            const uint64_t db = smem_desc_sw128(sa + A_BYTES);
+#pragma unroll
+            for (int t = 0; t < TM; ++t) {
+                const uint64_t da = smem_desc_sw128(sa + t * KTC_M * KT3_K);
+#pragma unroll
+                for (int kk = 0; kk < KT3_K / 32; ++kk)
+                    mma_i8(tmem + t * KTC_N, da + kk * 2, db + kk * 2, (s > 0 || kk > 0) ? 1u : 0u);
+            }
+            mma_commit(&empty[slot]);
+        }
+        mma_commit(&done);              // arrives once every MMA issued above has completed
+    }
+    __syncwarp();
+    if (!mbar_wait_bounded(&done, 0, wlim, a.status)) *vfail = 1;
+    tc_fence_after();
+    __syncthreads();
+    const bool ok = fail == 0;
+
+    // epilogue: warp w reads TMEM lanes 32 (w % 4) .., limb columns of half w / 4
+    for (int t = 0; t < TM; ++t) {
+        const long long row = row0 + t * KTC_M + 32 * (warp & 3) + lane;
+        const bool valid = ok && row < rows;
+        const ColStore<PACK, W64> out(a, valid ? first_row + row : 0);
+        const int cbase = (warp >> 2) * (KTC_N / 2);
+#pragma unroll 1
+        for (int c = cbase; c < cbase + KTC_N / 2; c += 32) {
+            uint32_t v[32];
+            tmem_ld32(tmem + t * KTC_N + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c, v);
+            tmem_wait_ld();
+            if (valid) out.store(col0 + c, v);
+            __syncwarp();
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(TM * KTC_N)));
+}
+
+template <int L, bool PACK, bool W64>
 __global__ void __launch_bounds__(KT2_THREADS, 1)
-    ks_tc2_kernel(const KsTcArgs a, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  int rows_fast) {
+    ks_tc2_kernel(const KsTcArgs a, const __grid_constant__ CUtensorMap tmB, int rows_fast) {
     constexpr int S = kt2_stages(L);
     constexpr int CH = 2 * L;                              // 16-byte K chunks per stage
     constexpr uint32_t A_BYTES = KTC_M * CH * 16;
@@ -501,7 +675,7 @@ __global__ void __launch_bounds__(KT2_THREADS, 1)
     }
     if (tid == 0) {
         for (int i = 0; i < S; ++i) {
-            mbar_init(&full[i], A_TMA ? 1u : 1u + 256u);
+            mbar_init(&full[i], 1u + 256u);
             mbar_init(&empty[i], 1);
         }
         mbar_init(&done, 1);
@@ -515,7 +689,7 @@ __global__ void __launch_bounds__(KT2_THREADS, 1)
 
     if (warp == 0) {
         if (lane == 0) {
-            // copies: B (and A) of stage s into slot s % S once the MMAs of
+            // copies: B of stage s into slot s % S once the MMAs of
             // stage s - S have released it
             int issued = 0;
             for (int s = 0; s < stages && !*vfail; ++s) {
@@ -525,23 +699,11 @@ __global__ void __launch_bounds__(KT2_THREADS, 1)
                     break;
                 }
                 unsigned char* st = smem_raw + (size_t)slot * (A_BYTES + B_BYTES);
-                mbar_arrive_expect_tx(&full[slot], B_BYTES + (A_TMA ? A_BYTES : 0u));
+                mbar_arrive_expect_tx(&full[slot], B_BYTES);
                 const int x0 = s * KTC_COEF * L;
-                if constexpr (SW) {
 #pragma unroll 1
-                    for (int kk = 0; kk < L; ++kk) {
-                        tma_load_2d(st + A_BYTES + kk * KTC_N * 32, &tmB, x0 + kk * 32, col0, &full[slot]);
-                        if constexpr (A_TMA)
-                            tma_load_2d(st + kk * KTC_M * 32, &tmA, x0 + kk * 32, (int)row0, &full[slot]);
-                    }
-                } else {
-#pragma unroll 1
-                    for (int c = 0; c < CH; ++c) {
-                        tma_load_2d(st + A_BYTES + c * KTC_N * 16, &tmB, x0 + c * 16, col0, &full[slot]);
-                        if constexpr (A_TMA)
-                            tma_load_2d(st + c * KTC_M * 16, &tmA, x0 + c * 16, (int)row0, &full[slot]);
-                    }
-                }
+                for (int kk = 0; kk < L; ++kk)
+                    tma_load_2d(st + A_BYTES + kk * KTC_N * 32, &tmB, x0 + kk * 32, col0, &full[slot]);
                 issued = s + 1;
             }
             // this thread's copies still in flight land before the CTA ends
@@ -561,10 +723,8 @@ __global__ void __launch_bounds__(KT2_THREADS, 1)
                 const uint32_t sb = sa + A_BYTES;
 #pragma unroll
                 for (int kk = 0; kk < L; ++kk) {   // K = 32 bytes = chunks 2 kk, 2 kk + 1
-                    const uint64_t da = (SW && A_TMA) ? smem_desc_sw32(sa + kk * KTC_M * 32)
-                                                      : smem_desc(sa + 2 * kk * KTC_M * 16, KTC_M * 16, 128);
-                    const uint64_t db = SW ? smem_desc_sw32(sb + kk * KTC_N * 32)
-                                           : smem_desc(sb + 2 * kk * KTC_N * 16, KTC_N * 16, 128);
+                    const uint64_t da = smem_desc(sa + 2 * kk * KTC_M * 16, KTC_M * 16, 128);
+                    const uint64_t db = smem_desc_sw32(sb + kk * KTC_N * 32);
                     mma_i8(tmem, da, db, (s > 0 || kk > 0) ? 1u : 0u);
                 }
                 mma_commit(&empty[slot]);
@@ -572,33 +732,31 @@ __global__ void __launch_bounds__(KT2_THREADS, 1)
             mma_commit(&done);              // arrives once every MMA issued above has completed
         }
     } else if (warp >= 4) {
-        if constexpr (!A_TMA) {
-            // digit producers: thread -> (row, half of the stage's 32 coefficients)
-            const int p = tid - 128, r = p & (KTC_M - 1), half = p >> 7;
-            const long long row = row0 + r;
-            for (int s = 0; s < stages && !*vfail; ++s) {
-                const int slot = s % S;
-                if (s >= S && !mbar_wait_bounded(&empty[slot], (uint32_t)(((s / S) + 1) & 1), wlim, a.status)) {
-                    *vfail = 1;
-                    break;
-                }
-                int8_t dig[16 * L];
-                if (row < a.B) {
-                    digits16<L, W64>(a.a_in, row * a.n_big + s * KTC_COEF + half * 16, a.log2_beta, dig);
-                } else {
-#pragma unroll
-                    for (int t = 0; t < 16 * L; ++t) dig[t] = 0;
-                }
-                unsigned char* base = smem_raw + (size_t)slot * (A_BYTES + B_BYTES) + r * 16;
-#pragma unroll
-                for (int c = 0; c < L; ++c) {
-                    uint4 v;
-                    memcpy(&v, dig + c * 16, 16);
-                    *reinterpret_cast<uint4*>(base + (half * L + c) * KTC_M * 16) = v;
-                }
-                fence_proxy_async_smem();
-                mbar_arrive_one(&full[slot]);
+        // digit producers: thread -> (row, half of the stage's 32 coefficients)
+        const int p = tid - 128, r = p & (KTC_M - 1), half = p >> 7;
+        const long long row = row0 + r;
+        for (int s = 0; s < stages && !*vfail; ++s) {
+            const int slot = s % S;
+            if (s >= S && !mbar_wait_bounded(&empty[slot], (uint32_t)(((s / S) + 1) & 1), wlim, a.status)) {
+                *vfail = 1;
+                break;
             }
+            int8_t dig[16 * L];
+            if (row < a.B) {
+                digits16<L, W64>(a.a_in, row * a.n_big + s * KTC_COEF + half * 16, a.log2_beta, dig);
+            } else {
+#pragma unroll
+                for (int t = 0; t < 16 * L; ++t) dig[t] = 0;
+            }
+            unsigned char* base = smem_raw + (size_t)slot * (A_BYTES + B_BYTES) + r * 16;
+#pragma unroll
+            for (int c = 0; c < L; ++c) {
+                uint4 v;
+                memcpy(&v, dig + c * 16, 16);
+                *reinterpret_cast<uint4*>(base + (half * L + c) * KTC_M * 16) = v;
+            }
+            fence_proxy_async_smem();
+            mbar_arrive_one(&full[slot]);
         }
     }
     if (!mbar_wait_bounded(&done, 0, wlim, a.status)) *vfail = 1;
@@ -672,31 +830,91 @@ static PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
     return fn;
 }
 
-// (rows, K) int8 matrix, row-major with K bytes per row; boxes of one 16-byte
-// K chunk x box_rows rows; rows past the end read as zero
-static int make_chunk_map(CUtensorMap* m, const void* base, long long K, long long rows, int box_rows, bool sw) {
+// (rows, K) int8 matrix, row-major with K bytes per row; boxes of box_k bytes
+// of box_rows rows; rows and columns past the end read as zero
+static int make_map(CUtensorMap* m, const void* base, long long K, long long rows, int box_rows, int box_k,
+                    CUtensorMapSwizzle swizzle) {
     const PFN_cuTensorMapEncodeTiled_v12000 enc = tma_encoder();
     if (!enc) return fail(TFHE_ERR_INTERNAL, "tensor-core contraction: cuTensorMapEncodeTiled unavailable");
     if ((reinterpret_cast<uintptr_t>(base) & 15) || K % 16)
         return fail(TFHE_ERR_INVALID_ARGUMENT, "tensor-core contraction: operand not 16-byte aligned");
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)K};
-    const cuuint32_t box[2] = {sw ? 32u : 16u, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
     const cuuint32_t es[2] = {1u, 1u};
     const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, es,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, sw ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? TFHE_OK : fail(TFHE_ERR_INTERNAL, "tensor-core contraction: tensor map encoding failed");
 }
 
-// TFHE_B200_TC_SW=0: 16-byte chunk copies without swizzling (for comparison)
-static bool tc_swizzle() {
-    static const bool on = [] {
-        const char* env = getenv("TFHE_B200_TC_SW");
-        return !(env && env[0] == '0');
-    }();
-    return on;
+constexpr int64_t KT3_DIGIT_BYTES = 192 << 20;         // digit matrix of one pass over the rows
+
+template <int TM, int S, bool PACK, bool W64>
+static int launch_tiles(const KsTcArgs& args, const int8_t* dig, long long first_row, long long rows, int parts,
+                        int part_steps, const CUtensorMap& tb, cudaStream_t stream) {
+    const long long rt = (rows + TM * KTC_M - 1) / (TM * KTC_M), ct = args.npad / KTC_N;
+    // the larger operand is streamed once: tiles sharing its slice run together
+    const bool rows_fast = (long long)args.npad > rows;
+    if ((rows_fast ? ct : rt) > 65535) return fail(TFHE_ERR_INVALID_ARGUMENT, "tensor-core contraction: too many tiles");
+    CUtensorMap ta;
+    TFHE_TRY(make_map(&ta, dig, (long long)args.n_big * args.l, rows, TM * KTC_M, KT3_K, CU_TENSOR_MAP_SWIZZLE_128B));
+    auto kern = ks_tc3_kernel<TM, S, PACK, W64>;
+    const size_t smem = kt3_smem(TM, S);
+    TFHE_TRY(tc_set_smem_once((const void*)kern, smem));
+    const dim3 grid = rows_fast ? dim3((unsigned)rt, (unsigned)ct, (unsigned)parts) : dim3((unsigned)ct, (unsigned)rt, (unsigned)parts);
+    count_launch();
+    kern<<<grid, KT3_THREADS, smem, stream>>>(args, ta, tb, rows_fast ? 1 : 0, first_row, rows, part_steps);
+    return check_cuda(cudaGetLastError(), "tensor-core contraction launch");
+}
+
+// *no_memory: the digit matrix found none, nothing was launched
+template <int L, bool PACK, bool W64>
+static int launch_l3(const KsTcArgs& args, cudaStream_t stream, bool* no_memory) {
+    const long long K = (long long)args.n_big * L;
+    const size_t word = W64 ? 8 : 4;
+    const long long chunk = std::min<long long>(args.B, std::max<long long>(2 * KTC_M, KT3_DIGIT_BYTES / K / (2 * KTC_M) * (2 * KTC_M)));
+    CUtensorMap tb;
+    TFHE_TRY(make_map(&tb, args.limbs, K, args.npad, KTC_N, KT3_K, CU_TENSOR_MAP_SWIZZLE_128B));
+    int8_t* dig = nullptr;
+    if (scratch_alloc((void**)&dig, (size_t)(chunk * K), stream) != cudaSuccess) {
+        cudaGetLastError();
+        *no_memory = true;
+        return TFHE_OK;
+    }
+    const long long sms = 148, ct = args.npad / KTC_N;
+    const int all_steps = (int)((K + KT3_K - 1) / KT3_K);
+    int rc = TFHE_OK;
+    for (long long first = 0; rc == TFHE_OK && first < args.B; first += chunk) {
+        const long long rows = std::min(chunk, args.B - first), words = rows * args.n_big;
+        const void* a_in = reinterpret_cast<const unsigned char*>(args.a_in) + (size_t)first * args.n_big * word;
+        count_launch();
+        tc_digits16_kernel<L, W64><<<(unsigned)std::min<long long>((words / 16 + 255) / 256, sms * 16), 256, 0, stream>>>(
+            a_in, words, args.log2_beta, dig);
+        rc = check_cuda(cudaGetLastError(), "digit matrix launch");
+        // 256-row tiles where their rounds (1.65 to 1.78 of the others' time
+        // each) are the shorter way (1024 LWEs: 241 against 257 us, 128: 81
+        // against 71); parts of at least eight K blocks where tiles are few
+        const long long t1 = (rows + KTC_M - 1) / KTC_M * ct, t2 = (rows + 2 * KTC_M - 1) / (2 * KTC_M) * ct;
+        const bool wide = (t2 + sms - 1) / sms * 5 <= (t1 + sms - 1) / sms * 3;
+        const int want = (int)std::max<long long>(1, std::min<long long>(sms / (wide ? t2 : t1), all_steps / 8));
+        const int part_steps = (all_steps + want - 1) / want, parts = (all_steps + part_steps - 1) / part_steps;
+        if (rc == TFHE_OK && !PACK && parts > 1) {
+            unsigned char* a_out = reinterpret_cast<unsigned char*>(args.a_out) + (size_t)first * args.n * word;
+            unsigned char* b_out = reinterpret_cast<unsigned char*>(args.b_out) + (size_t)first * word;
+            const unsigned char* b_in = reinterpret_cast<const unsigned char*>(args.b_in) + (size_t)first * word;
+            rc = check_cuda(cudaMemsetAsync(a_out, 0, (size_t)rows * args.n * word, stream), "key switch outputs");
+            if (rc == TFHE_OK && b_out != b_in)
+                rc = check_cuda(cudaMemcpyAsync(b_out, b_in, (size_t)rows * word, cudaMemcpyDeviceToDevice, stream),
+                                "key switch outputs");
+        }
+        if (rc == TFHE_OK)
+            rc = wide ? launch_tiles<2, 3, PACK, W64>(args, dig, first, rows, parts, part_steps, tb, stream)
+                      : launch_tiles<1, 4, PACK, W64>(args, dig, first, rows, parts, part_steps, tb, stream);
+    }
+    const int rc2 = check_cuda(cudaFreeAsync(dig, stream), "cudaFreeAsync(digits)");
+    return rc == TFHE_OK ? rc2 : rc;
 }
 
 template <int L, bool PACK, bool W64>
@@ -706,39 +924,25 @@ static int launch_l2(const KsTcArgs& args, cudaStream_t stream) {
     // the larger operand is streamed once: tiles sharing its slice run together
     const bool rows_fast = (long long)args.npad > args.B;
     if ((rows_fast ? ct : rt) > 65535) return fail(TFHE_ERR_INVALID_ARGUMENT, "tensor-core contraction: too many tiles");
-    CUtensorMap ta, tb;
-    memset(&ta, 0, sizeof(ta));
-    const bool sw = tc_swizzle();
-    int rc = make_chunk_map(&tb, args.limbs, K, args.npad, KTC_N, sw);
-    if (rc != TFHE_OK) return rc;
-    int8_t* dig = nullptr;
-    if (args.allow_alloc) {
-        rc = check_cuda(scratch_alloc((void**)&dig, (size_t)(args.B * K), stream), "working memory (digits)");
-        if (rc != TFHE_OK) return rc;
-        const long long words = args.B * (long long)args.n_big;
-        count_launch();
-        tc_digits_kernel<L, W64><<<(unsigned)std::min<long long>((words + 255) / 256, 148LL * 16), 256, 0, stream>>>(
-            args.a_in, args.B, args.n_big, args.log2_beta, dig);
-        rc = check_cuda(cudaGetLastError(), "digit matrix launch");
-        if (rc == TFHE_OK) rc = make_chunk_map(&ta, dig, K, args.B, KTC_M, sw);
+    CUtensorMap tb;
+    TFHE_TRY(make_map(&tb, args.limbs, K, args.npad, KTC_N, 32, CU_TENSOR_MAP_SWIZZLE_32B));
+    const size_t smem = (size_t)kt2_stages(L) * kt2_stage_bytes(L);
+    auto kern = ks_tc2_kernel<L, PACK, W64>;
+    TFHE_TRY(tc_set_smem_once((const void*)kern, smem));
+    const dim3 grid = rows_fast ? dim3((unsigned)rt, (unsigned)ct) : dim3((unsigned)ct, (unsigned)rt);
+    count_launch();
+    kern<<<grid, KT2_THREADS, smem, stream>>>(args, tb, rows_fast ? 1 : 0);
+    return check_cuda(cudaGetLastError(), "tensor-core contraction launch");
+}
+
+template <int L, bool PACK, bool W64>
+static int launch_pipelined(const KsTcArgs& args, cudaStream_t stream) {
+    if (args.allow_alloc && (long long)args.n_big * L >= KT3_K) {
+        bool no_memory = false;
+        const int rc = launch_l3<L, PACK, W64>(args, stream, &no_memory);
+        if (!no_memory) return rc;
     }
-    if (rc == TFHE_OK) {
-        const size_t smem = (size_t)kt2_stages(L) * kt2_stage_bytes(L);
-        auto kern = dig ? (sw ? ks_tc2_kernel<L, PACK, W64, true, true> : ks_tc2_kernel<L, PACK, W64, true, false>)
-                        : (sw ? ks_tc2_kernel<L, PACK, W64, false, true> : ks_tc2_kernel<L, PACK, W64, false, false>);
-        rc = tc_set_smem_once((const void*)kern, smem);
-        if (rc == TFHE_OK) {
-            const dim3 grid = rows_fast ? dim3((unsigned)rt, (unsigned)ct) : dim3((unsigned)ct, (unsigned)rt);
-            count_launch();
-            kern<<<grid, KT2_THREADS, smem, stream>>>(args, ta, tb, rows_fast ? 1 : 0);
-            rc = check_cuda(cudaGetLastError(), "tensor-core contraction launch");
-        }
-    }
-    if (dig) {
-        const int rc2 = check_cuda(cudaFreeAsync(dig, stream), "cudaFreeAsync(digits)");
-        if (rc == TFHE_OK) rc = rc2;
-    }
-    return rc;
+    return launch_l2<L, PACK, W64>(args, stream);
 }
 
 // TFHE_B200_TC_PIPE=0 selects the one-stage kernel (for comparison)
@@ -754,14 +958,14 @@ template <bool PACK, bool W64>
 static int launch_any(const KsTcArgs& args, cudaStream_t stream) {
     if (tc_pipelined()) {
         switch (args.l) {
-            case 1: return launch_l2<1, PACK, W64>(args, stream);
-            case 2: return launch_l2<2, PACK, W64>(args, stream);
-            case 3: return launch_l2<3, PACK, W64>(args, stream);
-            case 4: return launch_l2<4, PACK, W64>(args, stream);
-            case 5: return launch_l2<5, PACK, W64>(args, stream);
-            case 6: return launch_l2<6, PACK, W64>(args, stream);
-            case 7: return launch_l2<7, PACK, W64>(args, stream);
-            case 8: return launch_l2<8, PACK, W64>(args, stream);
+            case 1: return launch_pipelined<1, PACK, W64>(args, stream);
+            case 2: return launch_pipelined<2, PACK, W64>(args, stream);
+            case 3: return launch_pipelined<3, PACK, W64>(args, stream);
+            case 4: return launch_pipelined<4, PACK, W64>(args, stream);
+            case 5: return launch_pipelined<5, PACK, W64>(args, stream);
+            case 6: return launch_pipelined<6, PACK, W64>(args, stream);
+            case 7: return launch_pipelined<7, PACK, W64>(args, stream);
+            case 8: return launch_pipelined<8, PACK, W64>(args, stream);
             default: return fail(TFHE_ERR_INVALID_ARGUMENT, "tensor-core contraction: 1 <= l <= 8");
         }
     }
@@ -778,6 +982,7 @@ static int launch_any(const KsTcArgs& args, cudaStream_t stream) {
     }
 }
 
+// a_in 16-byte aligned (every caller checks)
 int launch_ks_tc(const KsTcArgs& args, cudaStream_t stream) {
     if (args.B == 0) return TFHE_OK;
     if (args.npad % KTC_N || args.n_big % KTC_COEF || (args.B + KTC_M - 1) / KTC_M > 65535)

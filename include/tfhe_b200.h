@@ -170,7 +170,8 @@ int tfhe_cuboot_merge(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32
  * (nn_tfhe/activation.py:148-162) = cuboot_merge(key_switch_LWE(h)).
  * a_in (batch, n_big), b_in (batch), lut (lut_count, 2, N)
  * -> out_a (batch, n_lut, N), out_b (batch, n_lut).
- * The key-switched intermediate is allocated stream-ordered on `stream`. */
+ * The key-switched intermediate and the key switch's digits (at most 192 MB)
+ * are allocated stream-ordered on `stream`. */
 int tfhe_pbs(const tfhe_keys* keys, const uint32_t* a_in, const uint32_t* b_in,
              const uint32_t* lut, int64_t lut_count, int32_t n_lut,
              uint32_t* out_a, uint32_t* out_b, int64_t batch, void* stream);
