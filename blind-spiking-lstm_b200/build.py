@@ -70,6 +70,7 @@ def build(force=False, jobs=None, verbose=False, extra_flags=()):
              ("ks_tc", os.path.join(CSRC, "ks_tc.cu"), []), ("torus64", os.path.join(CSRC, "torus64.cu"), []),
               ("trace_tree", os.path.join(CSRC, "trace_tree.cu"), []),
              ("br_fp32", os.path.join(CSRC, "br_fp32.cu"), [])]
+    units += [("br_share", os.path.join(CSRC, "br_share_inst.cu"), [])]
     units += [(f"br_mma{ref}", os.path.join(CSRC, "br_mma_inst.cu"), [f"-DBM_REF={ref}"]) for ref in (0, 1)]
     units += [(f"br_n{lg}", os.path.join(CSRC, "br_inst.cu"), [f"-DBR_LOGN={lg}"]) for lg in LOGNS]
     units += [(f"br64_n{lg}", os.path.join(CSRC, "br_inst64.cu"), [f"-DBR_LOGN={lg}"]) for lg in LOGNS]

@@ -569,6 +569,17 @@ static bool split_applies(int N, int L, int G, int M, long long B, bool reflayou
     return B <= split_resident_clusters(N, L, G, M, t64);
 }
 
+// Two ciphertexts per cluster of four CTAs (br_share.cuh), N = 2048, l_bs = 2,
+// four or eight patterns, for batches that fit one wave of such clusters but
+// not the forms above.  The same switches turn it off.
+static bool share_applies(int N, int L, int M, long long B, bool reflayout, int kr, const tfhe_tuning* tune, bool t64) {
+    const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
+    if (kr != 0 || reflayout || requested || N != 2048 || L != 2 || (M != 4 && M != 8) || B < 1 || !split_enabled() ||
+        !quad_enabled())
+        return false;
+    return B <= BS_K * resident_clusters(br_share_kernel_for(t64), BS_THREADS, br_share_smem(M), BS_C);
+}
+
 // the arguments of ciphertexts full .. B - 1 of a launch
 static BrArgs args_after(const BrArgs& args, long long full, int N) {
     BrArgs tail = args;
@@ -742,6 +753,9 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
     if (mma_takes(args, N, L, tune)) return launch_mma(args, N, L, stream, tune);
     if (const int S = cluster_form(N, L, args.G, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
         return launch_cluster_s(args, N, L, S, stream, tune);
+    if (share_applies(N, L, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
+        return launch_cluster(br_share_kernel_for(args.lwe_a64 != nullptr), BS_THREADS, br_share_smem(args.M), BS_C,
+                              (args.B + BS_K - 1) / BS_K, args, N, stream, tune, "blind rotation launch (shared key words)");
     if (split_applies(N, L, args.G, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
         return launch_split(args, N, L, stream, tune);
     if (!reflayout && kr == 0 && N == 2048 && L <= 2 &&

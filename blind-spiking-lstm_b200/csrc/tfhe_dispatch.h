@@ -5,6 +5,7 @@
 #include "br_cluster.cuh"
 #include "br_mma.cuh"
 #include "br_mma_cluster.cuh"
+#include "br_share.cuh"
 #include "br_split.cuh"
 #include "br_tm.cuh"
 #include "br_warp.cuh"
@@ -93,6 +94,9 @@ inline BrKernel br_tm_kernel_for(int logn, int L, bool t64) {
 BrKernel br_warp32_logn11(int NP);
 BrKernel br_warp64_logn11();
 inline BrKernel br_warp_kernel_for(bool t64, int NP) { return t64 ? br_warp64_logn11() : br_warp32_logn11(NP); }
+
+// two ciphertexts per cluster of four CTAs, N = 2048, l_bs = 2
+BrKernel br_share_kernel_for(bool t64);
 
 // the matrix-instruction kernels at N = 1024, l_bs 2 or 3, four or eight
 // patterns: four ciphertexts per CTA (C = 1) or per cluster of C = 2, 4 or 8

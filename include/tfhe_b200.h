@@ -134,7 +134,9 @@ int tfhe_keys_launch_shape(const tfhe_keys* keys, int64_t batch, int32_t* cipher
  * cluster form off); 0 for NULL keys.  At N = 1024, gadget base <= 2^8, l_bs 2
  * or 3 and collapse 2 or 3 the matrix-instruction form takes these batches
  * instead, four ciphertexts per cluster of eight, four or two CTAs (the same
- * switches turn those off).  Speed only: every form gives identical outputs. */
+ * switches turn those off).  At N = 2048, l_bs = 2 and collapse 2 or 3, most
+ * batches above the clusters of four (up to about 65) run two ciphertexts per
+ * cluster of four CTAs instead.  Speed only: every form gives identical outputs. */
 int32_t tfhe_keys_cluster_size(const tfhe_keys* keys, int64_t batch);
 int64_t tfhe_keys_device_bytes(const tfhe_keys* keys);
 

@@ -102,3 +102,25 @@ def test_dropin_n1024_matches_native_words(l_bs, log2_beta, collapse):
             want = keys.blind_rotate(a, torch.zeros(batch, dtype=torch.int32, device="cuda"), lut, 2)
             keys.set_tuning()
             assert torch.equal((got.to(torch.int64) & 0xFFFFFFFF), (want.to(torch.int64) & 0xFFFFFFFF)), (batch, shared)
+
+
+@pytest.mark.parametrize("torus", [32, 64])
+@pytest.mark.parametrize("collapse", [2, 3])
+def test_n2048_l2_small_batches_match_one_per_cta(torus, collapse):
+    """Four ciphertexts per cluster of eight or four CTAs: whole and partly
+    filled clusters, either side of each choice of form; 35 groups or more, so
+    that the rotation indices' window moves."""
+    word = torch.int32 if torus == 32 else torch.int64
+    if torus == 32:
+        p = ParamSet("n105_N2048", N=2048, n=35 * collapse, log2_beta_bs=15, l_bs=2, collapse=collapse, log2_beta_ks=4,
+                     l_ks=5, sigma_glwe=1.0, sigma_lwe=2.0 ** 15)
+        k = client.keygen(p, collapse)
+        keys = Keys.create(p, k.bsk, k.ksk_a, k.ksk_b)
+    else:
+        from tfhe_b200.torus64 import Keys64
+        p = client64.Params64("n105_N2048_q64", N=2048, n=35 * collapse, log2_beta_bs=13, l_bs=2, collapse=collapse,
+                              log2_beta_ks=4, l_ks=5, sigma_glwe=2.0 ** 17, sigma_lwe=2.0 ** 40)
+        keys = Keys64(client64.keygen(p, collapse))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for i, batch in enumerate([1, 3, 4, 5, sms // 4, sms // 2 - 2, sms // 2 + 1, sms - 20, sms]):
+        _compare(keys, p, word, p.n, batch, (1, 4)[i % 2], 10 * collapse + i)
