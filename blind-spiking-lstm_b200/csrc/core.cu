@@ -179,6 +179,11 @@ cudaError_t scratch_alloc(void** out, size_t bytes, cudaStream_t stream) {
     return pool ? cudaMallocFromPoolAsync(out, bytes, pool, stream) : cudaMallocAsync(out, bytes, stream);
 }
 
+void scratch_ready() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) scratch_pool(dev);
+}
+
 static void scratch_trim(int dev) {
     std::lock_guard<std::mutex> lk(g_pool_mu);
     if (dev >= 0 && dev < 64 && g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
@@ -190,6 +195,7 @@ const FftPlan* get_plan(int N) {
     std::lock_guard<std::mutex> lk(g_plan_mu);
     auto it = g_plans.find({dev, N});
     if (it != g_plans.end()) return it->second;
+    scratch_ready();
     std::vector<double2> qt, tw;
     std::vector<uint16_t> freq;
     build_tables(N, qt, tw, freq);
@@ -1195,7 +1201,11 @@ static int make_mma_key(tfhe_keys* k, cudaStream_t stream) {
     const tfhe_params& p = k->p;
     if (k->ring_kr > 0 || !mma_form(p.N, p.l_bs, k->M, p.log2_beta_bs, p.log2_q)) return TFHE_OK;
     const size_t bytes = (size_t)4 * k->G * k->M * p.l_bs * (p.N / 2) * sizeof(double2);
-    TFHE_TRY(check_cuda(cudaMalloc(&k->bsk_mma, bytes), "cudaMalloc(bsk, contraction layout)"));
+    if (cudaMalloc(&k->bsk_mma, bytes) != cudaSuccess) {     // no room for a second layout: the general kernels take these keys
+        cudaGetLastError();
+        k->bsk_mma = nullptr;
+        return TFHE_OK;
+    }
     k->bytes += (int64_t)bytes;
     const BmConvArgs ca{k->bsk, k->bsk_mma, k->G, k->M, p.l_bs};
     count_launch();

@@ -1017,6 +1017,7 @@ __global__ void limbs64_kernel(const unsigned long long* __restrict__ key, long 
 
 int build_limbs64(const unsigned long long* key, long long K, int cols, int npad, int8_t* limbs,
                   cudaStream_t stream) {
+    scratch_ready();
     const long long total = (long long)npad / 8 * K;
     const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 32);
     count_launch();
@@ -1045,6 +1046,7 @@ __global__ void packing_limbs_kernel(const uint32_t* __restrict__ ksp, int n_dim
 }
 
 int build_packing_limbs(const uint32_t* ksp, int n_dim, int l, int N, int8_t* limbs, cudaStream_t stream) {
+    scratch_ready();
     const long long total = 2LL * N * n_dim * l;
     const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 32);
     count_launch();

@@ -43,6 +43,9 @@ int fail(int code, const std::string& msg);
 int smem_attr_once(const void* kern, size_t smem);
 // stream-ordered working memory of one call (freed with cudaFreeAsync)
 cudaError_t scratch_alloc(void** out, size_t bytes, cudaStream_t stream);
+// makes the pool of the current device (keys and plans call it, so that the
+// first call that needs working memory may be one captured in a graph)
+void scratch_ready();
 int check_cuda(cudaError_t e, const char* what);
 
 // ----------------------------------------------------------------------------

@@ -77,7 +77,8 @@ const char* tfhe_last_error(void);
  *                (batch stride 0, mul_bootstrap.cuh:162-164)
  *   bsk          complex128, last six dims (G, 2, L, 2, M, N/2)
  *                (multiply.py:81-86); bsk_dims = those six extents
- *   all_rot_fft  complex128 (2N, N/2): row r = jax_fourier(X^r)
+ *   all_rot_fft  complex128 (2N, N/2): row r = jax_fourier(X^r); the kernels
+ *                that compute X^r from the index do not read it
  *   indices      int32 (batch, G, M)
  *   out          int64 (batch, 2, N)
  * degree in {128..4096}, l in {1..4}; other values -> INVALID_ARGUMENT.
