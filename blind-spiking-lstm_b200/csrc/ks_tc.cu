@@ -503,9 +503,10 @@ __global__ void __launch_bounds__(256) tc_digits16_kernel(const void* a_in, long
 // way) packing 2048 LWEs on the 64-bit torus took 1044 us, 1.3 int8 POP/s: TMA
 // works row by row, and 16-byte chunks had taken twice that again.  A copy here
 // brings rows of 128 bytes (128-byte swizzling, four MMA K steps) into a ring of
-// 48 KB slots: 486 us.  What is left is L2 traffic, (rows + columns) per tile
-// and digit; 256 x 256 tiles (two accumulators, all of TMEM, three 64 KB
-// slots) read a third less: 431 us, 3.2 POP/s, the measured bf16 rate twice.
+// 48 KB slots: 486 us.  256 x 256 tiles (two accumulators, all of TMEM, three
+// 64 KB slots) read a third less per digit: 431 us, 3.2 POP/s, twice the
+// measured bf16 rate, the tensor pipe 89% active.  Two 128-row CTAs per SM with
+// two slots each, so that one's epilogue overlaps, took 484 us.
 // The epilogue finds a row's place once, not a 64-bit division per output.
 //
 // Few tiles leave SMs idle, each one a serial sum over all digits: grid.z parts
