@@ -287,7 +287,7 @@ def run_engine(args, rank, world, local_rank, dist):
                 "outputs_equal_device_arm": not bool(e2e_diff)},
         "roofline": {"bound": "fp64", "achieved": round(achieved_tf, 3), "peak": round(peak_fp64, 3),
                      "unit": "TFLOP/s", "frac": round(achieved_tf / peak_fp64, 4), "traffic": traffic,
-                     "kernel": f"br_fp64_kernel<{p.N.bit_length() - 1},{p.l_bs}> (blind rotation + extraction)",
+                     "kernel": f"blind rotation + extraction launches, N = {p.N}, l_bs = {p.l_bs}",
                      "flops_per_pbs": int(fl), "launch_ms": round(br_ms, 3),
                      "peak_source": "FP64 FMA probe (tfhe_probe_fp64_fma) on this GPU; MEASURED_PEAKS.json "
                                     "holds no FP64 figure",
