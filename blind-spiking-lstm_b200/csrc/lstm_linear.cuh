@@ -48,15 +48,16 @@ __global__ void __launch_bounds__(LIN_NT) linear_kernel(const int32_t* __restric
 
     if (tid == 0) count = 0;
     __syncthreads();
-    for (int m = tid; m < N; m += LIN_NT) {                     // N is a multiple of 32: whole warps
+    // N is a multiple of 128, so every warp that enters is whole: full masks
+    for (int m = tid; m < N; m += LIN_NT) {
         int w[LIN_JT];
 #pragma unroll
         for (int jt = 0; jt < LIN_JT; ++jt) w[jt] = j0 + jt < J ? W[(long long)(j0 + jt) * N + m] : 0;
         const bool any = (w[0] | w[1] | w[2] | w[3]) != 0;
-        const unsigned vote = __ballot_sync(__activemask(), any);
+        const unsigned vote = __ballot_sync(0xffffffffu, any);
         int at = 0;
         if (lane == 0 && vote) at = atomicAdd(&count, __popc(vote));
-        at = __shfl_sync(__activemask(), at, 0) + __popc(vote & ((1u << lane) - 1u));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(vote & ((1u << lane) - 1u));
         if (any) {
             lm[at] = m;
             lw[at] = make_int4(w[0], w[1], w[2], w[3]);
