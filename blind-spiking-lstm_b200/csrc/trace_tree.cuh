@@ -244,10 +244,12 @@ __global__ void __launch_bounds__(TT_THREADS, 2) trace_tree_kernel(const TraceTr
         }
         __syncthreads();
 
-        // inner passes: the warp's block of the L digit polynomials
+        // inner passes: the warp's block of the L digit polynomials.  The 16 lanes
+        // of one polynomial exchange among themselves; an odd L leaves the upper
+        // half of the warp a round less
+        const unsigned mask = 0xffffu << (pl * 16);
 #pragma unroll 1
         for (int q = pl; q < L; q += 2) {
-            const unsigned mask = __activemask();
             double2 v[8], w[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) w[i] = node[i * TT_NODES + warp];

@@ -14,7 +14,7 @@ def code(name):
     return re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", text, flags=re.S))
 
 
-@pytest.mark.parametrize("name", ["lstm_linear.cuh"])
+@pytest.mark.parametrize("name", SOURCES)
 def test_warp_collectives_name_their_lanes(name):
     """__activemask() says which lanes happen to be converged, not which have to
     take part: a vote, shuffle or __syncwarp over it may run in parts."""
