@@ -499,7 +499,9 @@ static long long resident_clusters(BrKernel kern, int nt, size_t smem, int csize
     auto it = cache.find(key);
     if (it != cache.end()) return it->second;
     long long n = 0;
-    if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess) {
+    // (the attribute is only ever raised: a smaller key set's query must not
+    // take it from a larger one's launches)
+    if (smem_attr_once((const void*)kern, smem) == TFHE_OK) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(csize * std::max(1, sm_count())), 1, 1);
         cfg.blockDim = dim3(nt, 1, 1);

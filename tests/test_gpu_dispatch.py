@@ -1,0 +1,48 @@
+"""Which form a call runs, and that every form a key set reaches gives the
+one-ciphertext-per-CTA form's words, bit for bit."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from tfhe_b200.engine import Keys                           # noqa: E402
+from tfhe_b200.params import ParamSet                       # noqa: E402
+
+
+def _params(N, n, l_bs, log2_beta, collapse):
+    return ParamSet(f"n{n}_N{N}_c{collapse}", N=N, n=n, log2_beta_bs=log2_beta, l_bs=l_bs, collapse=collapse,
+                    log2_beta_ks=3, l_ks=2, sigma_glwe=1.0, sigma_lwe=1.0)
+
+
+def _keys(p, seed=0):
+    """Uniform words as keys: the forms compute on them as on real ones."""
+    rng = np.random.default_rng(seed)
+    words = lambda shape: rng.integers(0, 2 ** 32, size=shape, dtype=np.uint64).astype(np.uint32)
+    return Keys.create(p, words((2, 2, p.G * p.M, p.l_bs, p.N)), words((p.l_ks, p.N, p.n)), words((p.l_ks, p.N)))
+
+
+def _draw(shape, seed, dtype=torch.int32):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    info = torch.iinfo(dtype)
+    return torch.randint(info.min, info.max, shape, device="cuda", generator=g, dtype=dtype)
+
+
+def _same_as_one_per_cta(keys, batch, seed=0):
+    p = keys.params
+    a, b, lut = _draw((batch, p.n), seed), _draw((batch,), seed + 1), _draw((batch, 2, p.N), seed + 2)
+    got = keys.cuboot_merge(a, b, lut)
+    keys.set_tuning(ciphertexts_per_cta=1)
+    want = keys.cuboot_merge(a, b, lut)
+    keys.set_tuning()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), batch
+
+
+def test_key_sets_of_several_sizes_in_turn():
+    """A cluster kernel's shared memory grows with the number of groups and
+    patterns: a smaller key set in between leaves the larger one launchable."""
+    large, small = _keys(_params(1024, 120, 3, 9, 2)), _keys(_params(1024, 24, 3, 9, 2))
+    for keys in (large, small, large):
+        for batch in (1, 60):                                # one ciphertext per cluster of eight, per pair
+            _same_as_one_per_cta(keys, batch)
