@@ -1338,8 +1338,8 @@ int tfhe_keys_create(const tfhe_params* params, const uint32_t* bsk_coeff, const
     }
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     int rc = upload_bsk(k, bsk_coeff, sizeof(uint32_t), stream);
-    if (rc == TFHE_OK) rc = make_mma_key(k, stream);
     if (rc == TFHE_OK) rc = upload_ksk(k, ksk_a, ksk_b, stream);
+    if (rc == TFHE_OK) rc = make_mma_key(k, stream);         // last: it may go without memory
     if (rc != TFHE_OK) {
         keys_free(k);
         return rc;
@@ -1398,8 +1398,8 @@ int tfhe_keys_create_fourier(const tfhe_params* params, const double* bsk_ordere
                         "bsk upload");
     }
     if (rc == TFHE_OK) rc = check_cuda(cudaStreamSynchronize(stream), "bsk upload sync");
-    if (rc == TFHE_OK) rc = make_mma_key(k, stream);
     if (rc == TFHE_OK) rc = upload_ksk(k, ksk_a, ksk_b, stream);
+    if (rc == TFHE_OK) rc = make_mma_key(k, stream);         // last: it may go without memory
     if (rc != TFHE_OK) {
         keys_free(k);
         return rc;

@@ -22,6 +22,25 @@ def _keys(p, seed=0):
     return Keys.create(p, words((2, 2, p.G * p.M, p.l_bs, p.N)), words((p.l_ks, p.N, p.n)), words((p.l_ks, p.N)))
 
 
+class Hog:
+    """All of the GPU's memory but `leave` bytes, given back in steps."""
+
+    def __init__(self, leave):
+        torch.cuda.empty_cache()
+        self.held = [torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")]
+
+    def leave(self, nbytes):
+        del self.held[1:]
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        if free > nbytes:
+            self.held.append(torch.empty(free - nbytes, dtype=torch.uint8, device="cuda"))
+
+    def close(self):
+        self.held.clear()
+        torch.cuda.empty_cache()
+
+
 def _draw(shape, seed, dtype=torch.int32):
     g = torch.Generator(device="cuda")
     g.manual_seed(seed)
@@ -46,3 +65,36 @@ def test_key_sets_of_several_sizes_in_turn():
     for keys in (large, small, large):
         for batch in (1, 60):                                # one ciphertext per cluster of eight, per pair
             _same_as_one_per_cta(keys, batch)
+
+
+def test_keys_that_fit_without_the_second_layout():
+    """The second layout of a key (N = 1024, base <= 2^8) takes only memory that
+    the rest of the key set leaves: once a set fits, it fits with more memory
+    too, and without the layout it gives the same words."""
+    p = _params(1024, 120, 3, 7, 3).with_(l_ks=8)
+    both = _keys(p)
+    full = both.device_bytes()
+    both.close()
+    layout = p.bsk_bytes_fp64()
+    hog = Hog(full + (64 << 20))
+    fits, single = [], None
+    try:
+        for nbytes in range(layout, full + (32 << 20), 2 << 20):
+            hog.leave(nbytes)
+            try:
+                keys = _keys(p)
+            except Exception:
+                assert not fits, (nbytes, fits)
+                continue
+            fits.append(nbytes)
+            if keys.device_bytes() == full - layout:
+                single = keys
+            else:
+                assert keys.device_bytes() == full
+                keys.close()
+                break
+    finally:
+        hog.close()
+    assert single is not None
+    for batch in (1, 30, 60, 140, 300):
+        _same_as_one_per_cta(single, batch)
