@@ -97,8 +97,8 @@ __device__ __forceinline__ void st_async(uint32_t addr, double v, uint32_t bar) 
 }
 
 // wait for phase `parity` of a barrier that other CTAs complete; bounded as
-// mbar_wait_bounded
-__device__ __forceinline__ void bmc_wait(uint64_t* bar, uint32_t parity, long long limit, int* status) {
+// mbar_wait_bounded, false when it ran out
+__device__ __forceinline__ bool bmc_wait(uint64_t* bar, uint32_t parity, long long limit, int* status) {
     const long long t0 = clock64();
     for (;;) {
         uint32_t done;
@@ -109,15 +109,27 @@ __device__ __forceinline__ void bmc_wait(uint64_t* bar, uint32_t parity, long lo
             : "=r"(done)
             : "r"(smem_addr(bar)), "r"(parity)
             : "memory");
-        if (done) return;
+        if (done) return true;
         if (clock64() - t0 > limit) {
             if (status) atomicExch(status, TFHE_STATUS_WAIT_TIMEOUT);
-            return;
+            return false;
         }
     }
 }
 
-template <int L, int T, int C, bool REF>
+// After a wait that ran out: stores of other CTAs may still be on their way
+// into this CTA's shared memory although none is issued any more (a cluster
+// barrier lies behind), so the CTA stays for a few thousand times their latency
+// (about 1 ms)
+__device__ __forceinline__ void bmc_drain() {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) {
+    }
+}
+
+// LOST: the first CTA keeps back the digits of group 1 that the last one waits
+// for (the probe of what the kernel does then)
+template <int L, int T, int C, bool REF, bool LOST = false>
 __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrArgs args) {
     using S = BmcShape<L, C>;
     constexpr int LOGN = 10, LOGH = 9, P = 2 * L, K = BM_K, M = 4 * T;
@@ -233,7 +245,11 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
     };
 
     uint32_t phase = 0;                                              // of both barriers, one per group
-    for (long long iter = 0; iter < my_sets; ++iter) {
+    // A wait that runs out ends the loop at the CTA's next barrier, before it
+    // sends anything more; the others' waits for it then run out too, so a
+    // cluster ends within a few limits.  Its outputs are not written.
+    bool came = true, lost = false;
+    for (long long iter = 0; iter < my_sets && !lost; ++iter) {
         const long long ct0 = (cl + iter * ncl) * K;
         double acc_lo[8], acc_hi[8];
         {
@@ -371,6 +387,8 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
                     const uint32_t dst = peer_smem(rec + (size_t)(kc * P + bc) * PPC + (eo ^ ((eo >> 3) & 7) ^ x2),
                                                    (uint32_t)(bi / NA));
                     const double2 z = dig[at(pq, x, bi * 64 + e)];
+                    if constexpr (LOST)
+                        if (g == 1 && rank == 0 && bi / NA == C - 1) continue;
                     if constexpr (S::ASYNC) st_async(dst, z, peer_smem(&bars[0], (uint32_t)(bi / NA)));
                     else st_peer(dst, z);
                 }
@@ -379,7 +397,7 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
             if constexpr (S::STAGED < 1) load(ka, g, 0);
             if constexpr (S::STAGED < 2) load(kb, g, 1);
             // every digit of this CTA's points is here
-            if constexpr (S::ASYNC) bmc_wait(&bars[0], phase, args.wait_limit, args.status);
+            if constexpr (S::ASYNC) came = bmc_wait(&bars[0], phase, args.wait_limit, args.status);
             else cluster_barrier();
 
             // contraction of this warp's points, four at a time
@@ -426,7 +444,8 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
             }
             // every point of this CTA's outputs is here
             if constexpr (S::ASYNC) {
-                __syncthreads();
+                lost = __syncthreads_or(!came);
+                if (lost) break;
 #pragma unroll
                 for (int i = 0; i < 8 * PPC / BM_THREADS; ++i) {
                     const int o = (tid + i * BM_THREADS) / PPC, e = (tid + i * BM_THREADS) % PPC, p = rank * PPC + e;
@@ -434,7 +453,7 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
                     st_async(peer_smem(out + (size_t)out_poly(0, a) * H + (p ^ ((p >> 3) & 7) ^ a), (uint32_t)dst_rank),
                              gather[o * PPC + (e ^ ((e >> 3) & 7) ^ o)], peer_smem(&bars[1], (uint32_t)dst_rank));
                 }
-                bmc_wait(&bars[1], phase, args.wait_limit, args.status);
+                came = bmc_wait(&bars[1], phase, args.wait_limit, args.status);
             } else {
                 cluster_barrier();
             }
@@ -463,7 +482,12 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
 #pragma unroll
                 for (int j = 0; j < 8; ++j) poly[at(pq, x2, blk * 64 + t8 + 8 * j)] = v[j];
             }
-            __syncthreads();
+            if constexpr (S::ASYNC) {
+                lost = __syncthreads_or(!came);
+                if (lost) break;
+            } else {
+                __syncthreads();
+            }
 
             // last superstage, untwist, round, centred reduction (every level's threads)
             if (owner) {
@@ -486,6 +510,7 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
                 for (int n = 0; n < 8; ++n) acc_lo[n] = acc_hi[n] = 0.0;
             }
         }
+        if (lost) break;
         __syncthreads();                                             // dig and out are reused below
 
         if constexpr (REF) {
@@ -539,7 +564,9 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
         }
         __syncthreads();                                             // shared memory is reused by the next set
     }
+    if (lost) asm volatile("cp.async.wait_group 0;" ::: "memory");
     cluster_barrier();
+    if (lost) bmc_drain();
 }
 
 }  // namespace tfhe

@@ -33,6 +33,7 @@ BrKernel br_mma_ref(int L, int M, int C) { return pick(L, M, C); }
 BmRefConvKernel bm_ref_key() { return bm_ref_key_kernel; }
 #else
 BrKernel br_mma_native(int L, int M, int C) { return pick(L, M, C); }
+BrKernel br_mma_lost() { return br_mma_cluster_kernel<3, 2, 8, false, true>; }
 BmConvKernel bm_key() { return bm_key_kernel; }
 
 size_t br_mma_smem_for(int L, int M, int C) {

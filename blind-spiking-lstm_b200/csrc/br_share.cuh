@@ -135,7 +135,8 @@ __device__ __forceinline__ void bs_quarter16(double2 (&r)[4], int h, int h2, In 
             }
 }
 
-template <bool T64>
+// LOST as in br_mma_cluster_kernel
+template <bool T64, bool LOST = false>
 __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs args) {
     constexpr int LOGN = 11, LOGH = 10, N = 2048, H = 1024, P = 4, K = BS_K;
     constexpr int NB = BS_NB, MS = BS_STAGED;
@@ -224,6 +225,9 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
     copy(0);
 
     uint32_t phase = 0;                                              // of all barriers, one per group
+    // a wait that runs out ends the loop at the CTA's next barrier (see
+    // br_mma_cluster_kernel)
+    bool came = true, lost = false;
     for (int g = 0; g < args.G; ++g, phase ^= 1) {
         if (tid == 0) {
             mbar_arrive_expect_tx(&bars[0], DIGIT_BYTES);
@@ -301,9 +305,10 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
             const uint32_t dst_rank = (uint32_t)(w / NB);
             const uint32_t dst = peer_smem(rec, dst_rank), bar = peer_smem(&bars[0], dst_rank);
             const int row = ((w % NB) * K + ok) * P + 2 * lvl + oa;
+            const bool kept_back = LOST && g == 1 && rank == 0 && dst_rank == BS_C - 1;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
-                st_async(dst + (uint32_t)(rec_at(row, 2 * kk + h, j) * sizeof(double2)), r[bm_rev3(kk)], bar);
+                if (!kept_back) st_async(dst + (uint32_t)(rec_at(row, 2 * kk + h, j) * sizeof(double2)), r[bm_rev3(kk)], bar);
         }
         // the next two patterns' key words are on their way during the waits
         const double2* kg = args.bsk + (size_t)g * GROUP + (size_t)co * 2 * M * H * 2 + 2 * (size_t)u;
@@ -316,8 +321,8 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
         };
         load(MS);
         // every digit of this CTA's points is here, and the staged key words
-        mbar_wait_bounded(&bars[2], phase, args.wait_limit, args.status);
-        bmc_wait(&bars[0], phase, args.wait_limit, args.status);
+        came = mbar_wait_bounded(&bars[2], phase, args.wait_limit, args.status);
+        came &= bmc_wait(&bars[0], phase, args.wait_limit, args.status);
 
         // contraction: out = sum_m X^{r_m} sum_bc BSK[g, o, bc, m] DEC[bc]
         {
@@ -354,7 +359,8 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
 #pragma unroll
             for (int i = 0; i < K; ++i) gat[rec_at((cb * K + i) * 2 + co, ck2, cj)] = s[i];
         }
-        __syncthreads();
+        lost = __syncthreads_or(!came);
+        if (lost) break;
         if (g + 1 < args.G) {
             fence_proxy_async_smem();
             copy(g + 1);
@@ -373,7 +379,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
                 st_async(dst + (uint32_t)(out_at(rank * NB + b, 4 * kk + 2 * h2 + h, j) * sizeof(double2)),
                          r[((kk & 1) << 1) | (kk >> 1)], bar);
         }
-        bmc_wait(&bars[1], phase, args.wait_limit, args.status);
+        came = bmc_wait(&bars[1], phase, args.wait_limit, args.status);
 
         // inverse second superstage: butterfly (k0, n)
         if (lvl == 0) {
@@ -387,7 +393,11 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
 #pragma unroll
             for (int k1 = 0; k1 < 8; ++k1) op[out_at((k0 >> 1) * 2 + (k1 & 1), n, (k0 & 1) * 4 + (k1 >> 1))] = v[k1];
         }
-        __syncthreads();
+        lost = __syncthreads_or(!came);
+        if (lost) {
+            if (g + 1 < args.G) phase ^= 1;                          // of the key words on their way
+            break;
+        }
 
         // last superstage, untwist, round, centred reduction (both levels' threads)
         if (owner) {
@@ -411,6 +421,14 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
 #pragma unroll
             for (int n2 = 0; n2 < 8; ++n2) acc_lo[n2] = acc_hi[n2] = 0.0;
         }
+    }
+
+    if (lost) {
+        // this CTA's own bulk copies land (or have landed) before it ends
+        mbar_wait_bounded(&bars[2], phase, args.wait_limit, args.status);
+        cluster_barrier();
+        bmc_drain();
+        return;
     }
 
     // epilogue: rotate by -b~ and extract, as br_cluster_kernel (the CTA of

@@ -5,5 +5,6 @@
 namespace tfhe {
 
 BrKernel br_share_kernel_for(bool t64) { return t64 ? br_share_kernel<true> : br_share_kernel<false>; }
+BrKernel br_share_lost() { return br_share_kernel<false, true>; }
 
 }  // namespace tfhe

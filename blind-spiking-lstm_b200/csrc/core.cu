@@ -447,7 +447,7 @@ static int launch_cluster(BrKernel kern, int nt, size_t smem, int csize, long lo
     a.freq = pl->freq;
     a.K = 1;
     a.l2_prefetch = (tune && tune->l2_prefetch == 0) ? 0 : 1;
-    a.wait_limit = WAIT_LIMIT_CYCLES;
+    if (!a.wait_limit) a.wait_limit = LOOP_WAIT_LIMIT_CYCLES;
     a.status = device_status_word();
     if (!a.status) return fail(TFHE_ERR_INTERNAL, "device status word unavailable");
     cudaLaunchConfig_t cfg = {};
@@ -1484,12 +1484,10 @@ int tfhe_keyswitch(const tfhe_keys* keys, const uint32_t* a_in, const uint32_t* 
     return launch_ks(keys, a_in, b_in, a_out, b_out, batch, static_cast<cudaStream_t>(stream));
 }
 
-static int br_native(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32_t* lwe_b, const uint32_t* lut,
-                     int64_t lut_count, int32_t n_lut, uint32_t* acc_out, uint32_t* out_a, uint32_t* out_b,
-                     int64_t batch, cudaStream_t stream, int* status = nullptr) {
+static BrArgs native_args(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32_t* lwe_b, const uint32_t* lut,
+                          int64_t lut_count, int32_t n_lut, uint32_t* acc_out, uint32_t* out_a, uint32_t* out_b,
+                          int64_t batch) {
     const tfhe_params& p = keys->p;
-    if (n_lut < 1 || n_lut > p.N) return fail(TFHE_ERR_INVALID_ARGUMENT, "n_lut must be in [1, N]");
-    if (lut_count != 1 && lut_count != batch) return fail(TFHE_ERR_INVALID_ARGUMENT, "lut_count must be 1 or batch");
     BrArgs a{};
     a.bsk = keys->bsk;
     a.bsk_mma = keys->bsk_mma;
@@ -1508,7 +1506,38 @@ static int br_native(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32_
     a.acc_out = acc_out;
     a.out_a = out_a;
     a.out_b = out_b;
-    return launch_br(a, p.N, p.l_bs, false, keys->ring_kr, stream, status, &keys->tune);
+    return a;
+}
+
+static int br_native(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32_t* lwe_b, const uint32_t* lut,
+                     int64_t lut_count, int32_t n_lut, uint32_t* acc_out, uint32_t* out_a, uint32_t* out_b,
+                     int64_t batch, cudaStream_t stream, int* status = nullptr) {
+    const tfhe_params& p = keys->p;
+    if (n_lut < 1 || n_lut > p.N) return fail(TFHE_ERR_INVALID_ARGUMENT, "n_lut must be in [1, N]");
+    if (lut_count != 1 && lut_count != batch) return fail(TFHE_ERR_INVALID_ARGUMENT, "lut_count must be 1 or batch");
+    return launch_br(native_args(keys, lwe_a, lwe_b, lut, lut_count, n_lut, acc_out, out_a, out_b, batch), p.N, p.l_bs,
+                     false, keys->ring_kr, stream, status, &keys->tune);
+}
+
+int tfhe_probe_lost_message(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32_t* lwe_b, const uint32_t* lut,
+                            uint32_t* out_a, uint32_t* out_b, int64_t batch, int64_t limit_cycles, void* stream) {
+    TFHE_TRY(check_keys(keys));
+    const tfhe_params& p = keys->p;
+    if (batch < 1 || !lwe_a || !lwe_b || !lut || !out_a || !out_b)
+        return fail(TFHE_ERR_INVALID_ARGUMENT, "probe: NULL buffer or empty batch");
+    if (limit_cycles < 1 || limit_cycles > LOOP_WAIT_LIMIT_CYCLES)
+        return fail(TFHE_ERR_INVALID_ARGUMENT, "probe: limit out of range");
+    BrArgs a = native_args(keys, lwe_a, lwe_b, lut, 1, 1, nullptr, out_a, out_b, batch);
+    a.wait_limit = limit_cycles;
+    const bool mma = keys->bsk_mma && p.l_bs == 3 && keys->M == 8;
+    const bool share = keys->ring_kr == 0 && p.N == 2048 && p.l_bs == 2 && (keys->M == 4 || keys->M == 8);
+    if ((!mma && !share) || keys->G < 2)
+        return fail(TFHE_ERR_INVALID_ARGUMENT, "probe: no kernel of counted stores takes these keys");
+    if (mma)
+        return launch_cluster(br_mma_lost(), BM_THREADS, br_mma_smem_for(p.l_bs, keys->M, 8), 8, (batch + BM_K - 1) / BM_K, a,
+                              p.N, static_cast<cudaStream_t>(stream), &keys->tune, "probe launch");
+    return launch_cluster(br_share_lost(), BS_THREADS, br_share_smem(keys->M), BS_C, (batch + BS_K - 1) / BS_K, a, p.N,
+                          static_cast<cudaStream_t>(stream), &keys->tune, "probe launch");
 }
 
 int tfhe_blind_rotate(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32_t* lwe_b, const uint32_t* lut,

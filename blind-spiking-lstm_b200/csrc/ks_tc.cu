@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(KT3_THREADS, 1)
     const int step0 = (int)blockIdx.z * part_steps;
     const int steps = min(part_steps, (a.n_big * a.l + KT3_K - 1) / KT3_K - step0);
     volatile int* vfail = &fail;
-    const long long wlim = a.wait_limit < 200000000LL ? a.wait_limit : 200000000LL;
+    const long long wlim = a.wait_limit < LOOP_WAIT_LIMIT_CYCLES ? a.wait_limit : LOOP_WAIT_LIMIT_CYCLES;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(KT2_THREADS, 1)
     volatile int* vfail = &fail;
     // a stage's copies and MMAs take microseconds: a far shorter bound than
     // the caller's keeps a faulty launch from holding the GPU for long
-    const long long wlim = a.wait_limit < 200000000LL ? a.wait_limit : 200000000LL;
+    const long long wlim = a.wait_limit < LOOP_WAIT_LIMIT_CYCLES ? a.wait_limit : LOOP_WAIT_LIMIT_CYCLES;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),

@@ -97,6 +97,10 @@ inline BrKernel br_warp_kernel_for(bool t64, int NP) { return t64 ? br_warp64_lo
 
 // two ciphertexts per cluster of four CTAs, N = 2048, l_bs = 2
 BrKernel br_share_kernel_for(bool t64);
+// the same kernel, and the matrix-instruction one on clusters of eight (l_bs = 3,
+// eight patterns), with a message lost in group 1
+BrKernel br_share_lost();
+BrKernel br_mma_lost();
 
 // the matrix-instruction kernels at N = 1024, l_bs 2 or 3, four or eight
 // patterns: four ciphertexts per CTA (C = 1) or per cluster of C = 2, 4 or 8

@@ -38,6 +38,9 @@ int* device_status_word();
 void count_launch();
 // bound of every mbarrier wait, in clock cycles (about 2 s)
 constexpr long long WAIT_LIMIT_CYCLES = 4000000000LL;
+// the same for kernels that wait on other CTAs or copies in a loop and leave it
+// at the first wait that runs out (about 0.1 s)
+constexpr long long LOOP_WAIT_LIMIT_CYCLES = 200000000LL;
 int fail(int code, const std::string& msg);
 // the dynamic shared-memory attribute of a kernel, raised once per device and size
 int smem_attr_once(const void* kern, size_t smem);

@@ -236,6 +236,18 @@ int64_t tfhe_launch_count(void);
  * TFHE_DEVICE_TIMEOUT).  Synchronous. */
 int tfhe_probe_wait_timeout(int64_t limit_cycles, int32_t* waited_out);
 
+/* Diagnostics (no counterpart in the reference): the cuboot_merge of a batch
+ * (n_lut 1, one LUT) by the cluster kernel whose CTAs count the stores they
+ * get, with one message left out in every cluster and waits limited to
+ * limit_cycles.  The CTAs that miss it give up, then those that wait for
+ * them; the kernel ends within a few limits, leaves the outputs alone and
+ * records TFHE_DEVICE_TIMEOUT.  Keys that run such a kernel only (N = 1024
+ * with l_bs 3 and eight patterns at base <= 2^8, N = 2048 with l_bs 2 and
+ * four or eight patterns). */
+int tfhe_probe_lost_message(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32_t* lwe_b,
+                            const uint32_t* lut, uint32_t* out_a, uint32_t* out_b, int64_t batch,
+                            int64_t limit_cycles, void* stream);
+
 /* tfhe_pbs from HOST buffers (pinned, for overlap): the batch is processed
  * in chunks of `chunk` ciphertexts (0: automatic); each chunk's upload,
  * compute and download run on separate streams so the copies overlap the

@@ -98,3 +98,35 @@ def test_keys_that_fit_without_the_second_layout():
     assert single is not None
     for batch in (1, 30, 60, 140, 300):
         _same_as_one_per_cta(single, batch)
+
+
+@pytest.mark.parametrize("N,n,l_bs,log2_beta,collapse", [(1024, 630, 3, 7, 3), (2048, 742, 2, 15, 2)])
+@pytest.mark.parametrize("clusters", [1, 5])
+def test_a_lost_message_ends_the_cluster(N, n, l_bs, log2_beta, collapse, clusters):
+    """One message of group 1 never arrives.  The waits for it run out, then those
+    for the CTAs that gave up, and the kernel ends: three limits of 1 ms and the
+    stay of 1 ms behind them at most, 10 ms with the launch (to run out in every
+    group would take hundreds).  Outputs stay, the status says so, the keys work."""
+    import ctypes
+    from tfhe_b200 import _lib
+    lib = _lib.load()
+    keys = _keys(_params(N, n, l_bs, log2_beta, collapse))
+    batch = clusters * (4 if N == 1024 else 2)
+    a, b, lut = _draw((batch, n), 1), _draw((batch,), 2), _draw((1, 2, N), 3)
+    out_a = torch.full((batch, 1, N), 77, dtype=torch.int32, device="cuda")
+    out_b = torch.full((batch, 1), 77, dtype=torch.int32, device="cuda")
+    _same_as_one_per_cta(keys, batch)
+    st = ctypes.c_int32()
+    _lib.check(lib.tfhe_device_status(ctypes.byref(st), 1))
+    t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    p = lambda x: ctypes.c_void_p(x.data_ptr())
+    t0.record()
+    _lib.check(lib.tfhe_probe_lost_message(keys.handle, p(a), p(b), p(lut), p(out_a), p(out_b), batch, 1_900_000,
+                                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    t1.record()
+    torch.cuda.synchronize()
+    _lib.check(lib.tfhe_device_status(ctypes.byref(st), 1))
+    assert st.value == 1
+    assert t0.elapsed_time(t1) < 10.0
+    assert bool((out_a == 77).all()) and bool((out_b == 77).all())
+    _same_as_one_per_cta(keys, batch)
