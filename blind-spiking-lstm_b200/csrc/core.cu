@@ -433,9 +433,24 @@ static bool split_enabled() {
     return on;
 }
 
-// `clusters` clusters of `csize` CTAs
-static int launch_cluster(BrKernel kern, int nt, size_t smem, int csize, long long clusters, const BrArgs& args, int N,
-                          cudaStream_t stream, const tfhe_tuning* tune, const char* what) {
+// The launches of one blind rotation: launch_br fills a caller's list instead
+// of launching, so what is reported is what would run
+struct BrPlan {
+    static constexpr int MAX = 8;
+    tfhe_launch at[MAX];
+    int n = 0;
+    int add(long long ciphertexts, int per_unit, int ctas) {
+        if (n < MAX) at[n] = tfhe_launch{ciphertexts, per_unit, ctas};
+        ++n;
+        return TFHE_OK;
+    }
+};
+
+// clusters of `csize` CTAs, K ciphertexts each
+static int launch_cluster(BrKernel kern, int nt, size_t smem, int csize, int K, const BrArgs& args, int N,
+                          cudaStream_t stream, const tfhe_tuning* tune, const char* what, BrPlan* plan = nullptr) {
+    if (plan) return plan->add(args.B, K, csize);
+    const long long clusters = (args.B + K - 1) / K;
     int per_sm = 1;
     TFHE_TRY(prepare_kernel((const void*)kern, nt, smem, &per_sm));
     BrArgs a = args;
@@ -466,22 +481,24 @@ static int launch_cluster(BrKernel kern, int nt, size_t smem, int csize, long lo
     return check_cuda(cudaLaunchKernelEx(&cfg, kern, a), what);
 }
 
-static int launch_split(const BrArgs& args, int N, int L, cudaStream_t stream, const tfhe_tuning* tune) {
+static int launch_split(const BrArgs& args, int N, int L, cudaStream_t stream, const tfhe_tuning* tune, BrPlan* plan) {
     const bool t64 = args.lwe_a64 != nullptr;
     BrKernel kern = br_split_kernel_for(ilog2(N), L, t64);
     if (!kern) return fail(TFHE_ERR_INVALID_ARGUMENT, "unsupported degree / levels");
-    return launch_cluster(kern, BR_SPLIT_THREADS, br_split_smem(N, L, args.G, args.M, br_table_bytes(N)), 2, args.B,
-                          args, N, stream, tune, "blind rotation launch (cluster pair)");
+    return launch_cluster(kern, BR_SPLIT_THREADS, br_split_smem(N, L, args.G, args.M, br_table_bytes(N)), 2, 1,
+                          args, N, stream, tune, "blind rotation launch (cluster pair)", plan);
 }
 
 // one ciphertext per cluster of 2 S CTAs (br_cluster.cuh)
-static int launch_cluster_s(const BrArgs& args, int N, int L, int S, cudaStream_t stream, const tfhe_tuning* tune) {
+static int launch_cluster_s(const BrArgs& args, int N, int L, int S, cudaStream_t stream, const tfhe_tuning* tune,
+                            BrPlan* plan) {
     const bool t64 = args.lwe_a64 != nullptr;
     BrKernel kern = br_cluster_kernel_for(ilog2(N), L, t64, S);
     if (!kern) return fail(TFHE_ERR_INVALID_ARGUMENT, "unsupported degree / levels");
     return launch_cluster(kern, BR_CLUSTER_THREADS, br_cluster_smem(N, L, args.G, args.M, br_table_bytes(N), S),
-                          2 * S, args.B, args, N, stream, tune,
-                          S == 4 ? "blind rotation launch (cluster of eight)" : "blind rotation launch (cluster of four)");
+                          2 * S, 1, args, N, stream, tune,
+                          S == 4 ? "blind rotation launch (cluster of eight)" : "blind rotation launch (cluster of four)",
+                          plan);
 }
 
 // clusters of `csize` CTAs of this kernel that can be resident at once (a
@@ -623,7 +640,8 @@ static bool tm_default() {
 }
 
 static int launch_tm(const BrArgs& args, int N, int L, cudaStream_t stream, const tfhe_tuning* tune,
-                     long long full) {
+                     long long full, BrPlan* plan) {
+    if (plan) return plan->add(full, 3, 1);
     const bool t64 = args.lwe_a64 != nullptr;
     BrKernel kern = br_tm_kernel_for(ilog2(N), L, t64);
     if (!kern) return fail(TFHE_ERR_INVALID_ARGUMENT, "unsupported degree / levels");
@@ -688,7 +706,8 @@ static long long mma_cluster_capacity(int L, int M, int C, bool ref) {
 // that hold it in one wave, or a partly filled round (n=630, cycles per group:
 // four per SM 38k, clusters of two 27k for two per SM, of four 18.5k for about
 // one per SM, of eight 11.3k).
-static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, const tfhe_tuning* tune) {
+static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, const tfhe_tuning* tune,
+                      BrPlan* plan = nullptr) {
     const bool ref = args.ct_init != nullptr;
     const long long round = (long long)BM_K * std::max(1, sm_count());
     const long long full = args.B / round * round;
@@ -697,7 +716,9 @@ static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, con
     for (int c : {2, 4, 8})
         if (rest > 0 && rest <= mma_cluster_capacity(L, args.M, c, ref)) C = c;
     const long long head = C ? full : args.B;
-    if (head > 0) {
+    if (head > 0 && plan) {
+        plan->add(head, BM_K, 1);
+    } else if (head > 0) {
         BrKernel kern = br_mma_kernel_for(L, args.M, 1, ref);
         const size_t smem = br_mma_smem_for(L, args.M, 1);
         int per_sm = 1;
@@ -716,9 +737,9 @@ static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, con
         TFHE_TRY(check_cuda(cudaGetLastError(), "blind rotation launch (matrix instruction)"));
     }
     if (!C) return TFHE_OK;
-    return launch_cluster(br_mma_kernel_for(L, args.M, C, ref), BM_THREADS, br_mma_smem_for(L, args.M, C), C,
-                          (rest + BM_K - 1) / BM_K, full ? args_after(args, full, N) : args, N, stream, tune,
-                          "blind rotation launch (matrix instruction, cluster)");
+    return launch_cluster(br_mma_kernel_for(L, args.M, C, ref), BM_THREADS, br_mma_smem_for(L, args.M, C), C, BM_K,
+                          full ? args_after(args, full, N) : args, N, stream, tune,
+                          "blind rotation launch (matrix instruction, cluster)", plan);
 }
 
 // Ciphertexts of a batch that go to the four-per-CTA kernel in automatic
@@ -735,7 +756,8 @@ static long long warp_four_share(int N, int L, int G, int M, long long B, bool r
     return B - full > (M <= 4 ? 3 : 2) * sms ? B : full;
 }
 
-static int launch_warp_four(const BrArgs& args, int N, cudaStream_t stream, const tfhe_tuning* tune) {
+static int launch_warp_four(const BrArgs& args, int N, cudaStream_t stream, const tfhe_tuning* tune, BrPlan* plan) {
+    if (plan) return plan->add(args.B, 4, 1);
     BrKernel kern = br_warp_kernel_for(args.lwe_a64 != nullptr, 2);
     const size_t smem = br_warp_smem(2, args.G, args.M);
     int per_sm = 1;
@@ -755,36 +777,36 @@ static int launch_warp_four(const BrArgs& args, int N, cudaStream_t stream, cons
 }
 
 static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStream_t stream,
-                     int* status = nullptr, const tfhe_tuning* tune = nullptr) {
+                     int* status = nullptr, const tfhe_tuning* tune = nullptr, BrPlan* plan = nullptr) {
     const int logn = ilog2(N);
     const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
-    if (mma_takes(args, N, L, tune)) return launch_mma(args, N, L, stream, tune);
+    if (mma_takes(args, N, L, tune)) return launch_mma(args, N, L, stream, tune, plan);
     if (const int S = cluster_form(N, L, args.G, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
-        return launch_cluster_s(args, N, L, S, stream, tune);
+        return launch_cluster_s(args, N, L, S, stream, tune, plan);
     if (share_applies(N, L, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
         return launch_cluster(br_share_kernel_for(args.lwe_a64 != nullptr), BS_THREADS, br_share_smem(args.M), BS_C,
-                              (args.B + BS_K - 1) / BS_K, args, N, stream, tune, "blind rotation launch (shared key words)");
+                              BS_K, args, N, stream, tune, "blind rotation launch (shared key words)", plan);
     if (split_applies(N, L, args.G, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr))
-        return launch_split(args, N, L, stream, tune);
+        return launch_split(args, N, L, stream, tune, plan);
     if (!reflayout && kr == 0 && N == 2048 && L <= 2 &&
         ((tune && tune->ciphertexts_per_cta == 3) || (!requested && tm_default())) &&
         br_tm_smem(N, L, 3, args.M, br_table_bytes(N)) <= (size_t)max_smem_optin()) {
         const long long round = 3LL * sm_count();
         const long long full = (args.B / round) * round;
         if (full > 0) {
-            TFHE_TRY(launch_tm(args, N, L, stream, tune, full));
+            TFHE_TRY(launch_tm(args, N, L, stream, tune, full, plan));
             if (full == args.B) return TFHE_OK;
             tfhe_tuning rest_tune = tune ? *tune : tfhe_tuning{0, -1, -1, -1, -1};
             if (rest_tune.ciphertexts_per_cta == 3) rest_tune.ciphertexts_per_cta = 0;
-            return launch_br(args_after(args, full, N), N, L, reflayout, kr, stream, status, &rest_tune);
+            return launch_br(args_after(args, full, N), N, L, reflayout, kr, stream, status, &rest_tune, plan);
         }
     }
     if (const long long four = warp_four_share(N, L, args.G, args.M, args.B, reflayout, kr, tune)) {
         BrArgs head = args;
         head.B = four;
-        TFHE_TRY(launch_warp_four(head, N, stream, tune));
+        TFHE_TRY(launch_warp_four(head, N, stream, tune, plan));
         if (four == args.B) return TFHE_OK;
-        return launch_br(args_after(args, four, N), N, L, reflayout, kr, stream, status, tune);
+        return launch_br(args_after(args, four, N), N, L, reflayout, kr, stream, status, tune, plan);
     }
     const BrShape sh = kr > 0 ? ring_shape(N, L, args.M)
                               : br_shape(N, L, args.M, args.B, tune ? tune->ciphertexts_per_cta : 0, !reflayout);
@@ -848,12 +870,17 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
         if (rest > 0 && rest <= sm_count()) {
             BrArgs head = args;
             head.B = full;
-            count_launch();
-            kern<<<(unsigned)grid, nt, smem, stream>>>(head);
-            TFHE_TRY(check_cuda(cudaGetLastError(), "blind rotation launch"));
-            return launch_br(args_after(args, full, N), N, L, reflayout, 0, stream, status, tune);
+            if (plan) {
+                plan->add(full, sh.K, 1);
+            } else {
+                count_launch();
+                kern<<<(unsigned)grid, nt, smem, stream>>>(head);
+                TFHE_TRY(check_cuda(cudaGetLastError(), "blind rotation launch"));
+            }
+            return launch_br(args_after(args, full, N), N, L, reflayout, 0, stream, status, tune, plan);
         }
     }
+    if (plan) return plan->add(args.B, sh.K, 1);
     count_launch();
     kern<<<(unsigned)grid, nt, smem, stream>>>(args);
     return check_cuda(cudaGetLastError(), "blind rotation launch");
@@ -1534,9 +1561,9 @@ int tfhe_probe_lost_message(const tfhe_keys* keys, const uint32_t* lwe_a, const 
     if ((!mma && !share) || keys->G < 2)
         return fail(TFHE_ERR_INVALID_ARGUMENT, "probe: no kernel of counted stores takes these keys");
     if (mma)
-        return launch_cluster(br_mma_lost(), BM_THREADS, br_mma_smem_for(p.l_bs, keys->M, 8), 8, (batch + BM_K - 1) / BM_K, a,
-                              p.N, static_cast<cudaStream_t>(stream), &keys->tune, "probe launch");
-    return launch_cluster(br_share_lost(), BS_THREADS, br_share_smem(keys->M), BS_C, (batch + BS_K - 1) / BS_K, a, p.N,
+        return launch_cluster(br_mma_lost(), BM_THREADS, br_mma_smem_for(p.l_bs, keys->M, 8), 8, BM_K, a, p.N,
+                              static_cast<cudaStream_t>(stream), &keys->tune, "probe launch");
+    return launch_cluster(br_share_lost(), BS_THREADS, br_share_smem(keys->M), BS_C, BS_K, a, p.N,
                           static_cast<cudaStream_t>(stream), &keys->tune, "probe launch");
 }
 
@@ -1757,6 +1784,24 @@ int32_t tfhe_keys_cluster_size(const tfhe_keys* keys, int64_t batch) {
     if (const int S = cluster_form(p.N, p.l_bs, keys->G, keys->M, batch, false, keys->ring_kr, &keys->tune, t64))
         return 2 * S;
     return split_applies(p.N, p.l_bs, keys->G, keys->M, batch, false, keys->ring_kr, &keys->tune, t64) ? 2 : 1;
+}
+
+int32_t tfhe_keys_launches(const tfhe_keys* keys, int64_t batch, tfhe_launch* launches, int32_t capacity) {
+    if (!keys || batch < 0 || capacity < 0 || (capacity > 0 && !launches)) return -1;
+    if (batch == 0) return 0;
+    const tfhe_params& p = keys->p;
+    // what br_native and br_native64 hand to launch_br, without buffers
+    BrArgs a = native_args(keys, nullptr, nullptr, nullptr, 1, 1, nullptr, nullptr, nullptr, batch);
+    if (p.log2_q == 64) {
+        a.bsk_mma = nullptr;
+        a.log2_q = 64;
+        a.lwe_a64 = reinterpret_cast<const unsigned long long*>(keys->bsk);      // marks the torus, not read
+    }
+    BrPlan plan;
+    if (launch_br(a, p.N, p.l_bs, false, p.log2_q == 64 ? 0 : keys->ring_kr, nullptr, nullptr, &keys->tune, &plan) != TFHE_OK)
+        return -1;
+    for (int i = 0; i < std::min<int>(plan.n, std::min<int>(capacity, BrPlan::MAX)); ++i) launches[i] = plan.at[i];
+    return plan.n;
 }
 
 int64_t tfhe_launch_count(void) { return launch_count(); }

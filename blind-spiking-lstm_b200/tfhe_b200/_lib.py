@@ -34,6 +34,11 @@ class TfheParams(ctypes.Structure):
                 ("N", "n", "n_big", "log2_beta_bs", "l_bs", "collapse", "log2_beta_ks", "l_ks", "log2_q")]
 
 
+class TfheLaunch(ctypes.Structure):
+    _fields_ = [("ciphertexts", ctypes.c_int64), ("ciphertexts_per_unit", ctypes.c_int32),
+                ("ctas_per_unit", ctypes.c_int32)]
+
+
 _P = ctypes.c_void_p
 _I32 = ctypes.c_int32
 _I64 = ctypes.c_int64
@@ -48,6 +53,7 @@ SIGNATURES = {
     "tfhe_keys_destroy": (None, [_P]),
     "tfhe_keys_set_tuning": (ctypes.c_int, [_P, ctypes.POINTER(TfheTuning)]),
     "tfhe_keys_cluster_size": (ctypes.c_int32, [_P, _I64]),
+    "tfhe_keys_launches": (_I32, [_P, _I64, ctypes.POINTER(TfheLaunch), _I32]),
     "tfhe_keys_launch_shape": (ctypes.c_int, [_P, _I64, ctypes.POINTER(_I32), ctypes.POINTER(_I32),
                                               ctypes.POINTER(_I64)]),
     "tfhe_keys_device_bytes": (_I64, [_P]),
@@ -129,6 +135,15 @@ def check(status: int) -> None:
     if status != 0:
         msg = load().tfhe_last_error()
         raise TFHEError(int(status), msg.decode() if msg else "")
+
+
+def keys_launches(handle, batch: int) -> list:
+    """tfhe_keys_launches as (ciphertexts, ciphertexts per unit, CTAs per unit)."""
+    at = (TfheLaunch * 8)()
+    n = load().tfhe_keys_launches(handle, int(batch), at, 8)
+    if n < 0:
+        raise ValueError(f"no launches for a batch of {batch}")
+    return [(x.ciphertexts, x.ciphertexts_per_unit, x.ctas_per_unit) for x in at[:n]]
 
 
 def version() -> str:

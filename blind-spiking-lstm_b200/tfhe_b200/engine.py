@@ -149,10 +149,14 @@ class Keys:
         return k.value, nt.value, sm.value
 
     def cluster_size(self, batch: int) -> int:
-        """CTAs per ciphertext of a batch's blind rotation: 8, 4 or 2 where
-        one ciphertext runs on a cluster of that many CTAs (small batches),
-        else 1."""
+        """CTAs per ciphertext in the forms of one ciphertext per cluster (8, 4
+        or 2 by batch size, else 1); `launches` says what a batch runs."""
         return int(_lib.load().tfhe_keys_cluster_size(self.handle, int(batch)))
+
+    def launches(self, batch: int) -> list:
+        """The launches of a batch's blind rotation in order, each (ciphertexts,
+        ciphertexts per CTA or cluster, CTAs per cluster; 1: no cluster)."""
+        return _lib.keys_launches(self.handle, batch)
 
     def device_bytes(self) -> int:
         return int(_lib.load().tfhe_keys_device_bytes(self.handle))

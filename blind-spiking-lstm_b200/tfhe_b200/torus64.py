@@ -92,9 +92,13 @@ class Keys64:
         self.ks_tensor_cores = int(ks_tensor_cores)
 
     def cluster_size(self, batch: int) -> int:
-        """CTAs per ciphertext of a batch's blind rotation (8, 4 or 2: one
-        ciphertext per cluster of that many CTAs; 1: several per CTA)."""
+        """CTAs per ciphertext in the forms of one ciphertext per cluster (8, 4
+        or 2 by batch size, else 1); `launches` says what a batch runs."""
         return int(_lib.load().tfhe_keys_cluster_size(self.handle, int(batch)))
+
+    def launches(self, batch: int) -> list:
+        """As `engine.Keys.launches`."""
+        return _lib.keys_launches(self.handle, batch)
 
     def close(self):
         if getattr(self, "handle", None):

@@ -125,20 +125,31 @@ int tfhe_keys_set_tuning(tfhe_keys* keys, const tfhe_tuning* tuning);
 int tfhe_keys_launch_shape(const tfhe_keys* keys, int64_t batch, int32_t* ciphertexts_per_cta,
                            int32_t* threads, int64_t* shared_bytes);
 
-/* CTAs per ciphertext a batch's blind rotation takes: 8 where one
- * ciphertext runs on a cluster of eight CTAs (N = 1024 or 2048, collapse
- * <= 3, at N = 1024 collapse >= 2; batches of at most an eighth of the SM
- * count; TFHE_B200_OCTET=0 turns it off), 4 on a cluster of four (N = 1024
- * or 2048, at most a quarter;
- * TFHE_B200_QUAD=0 turns both off), 2 on a cluster of two (at most half the
- * SM count), else 1 (automatic shapes only; TFHE_B200_SPLIT=0 turns every
- * cluster form off); 0 for NULL keys.  At N = 1024, gadget base <= 2^8, l_bs 2
- * or 3 and collapse 2 or 3 the matrix-instruction form takes these batches
- * instead, four ciphertexts per cluster of eight, four or two CTAs (the same
- * switches turn those off).  At N = 2048, l_bs = 2 and collapse 2 or 3, most
- * batches above the clusters of four (up to about 65) run two ciphertexts per
- * cluster of four CTAs instead.  Speed only: every form gives identical outputs. */
+/* CTAs per ciphertext in the forms that run one ciphertext per cluster: 8
+ * for batches of at most an eighth of the SM count (N = 1024 or 2048,
+ * collapse <= 3, at N = 1024 collapse >= 2; TFHE_B200_OCTET=0 turns it off),
+ * 4 for at most a quarter (TFHE_B200_QUAD=0 turns both off), 2 for at most
+ * half the SM count, else 1 (automatic shapes only; TFHE_B200_SPLIT=0 turns
+ * every cluster form off); 0 for NULL keys.  Forms of several ciphertexts per
+ * cluster take some of these batches and others: tfhe_keys_launches says
+ * what runs.  Speed only: every form gives identical outputs. */
 int32_t tfhe_keys_cluster_size(const tfhe_keys* keys, int64_t batch);
+
+/* The launches of a batch's blind rotation, in order: `ciphertexts` of the
+ * batch in units of `ciphertexts_per_unit`, each on a cluster of
+ * `ctas_per_unit` CTAs (1: no cluster; a launch of fewer CTAs than units
+ * loops).  Writes at most `capacity` of them and returns their number, -1
+ * for invalid arguments.  At N = 1024, base <= 2^8, l_bs 2 or 3 and collapse
+ * 2 or 3 the matrix-instruction forms run four ciphertexts per CTA or per
+ * cluster of eight, four or two; at N = 2048 and l_bs = 2 there are two per
+ * cluster of four, and two or four per CTA (no counterpart in the reference;
+ * TFHE_B200_QUAD, _OCTET and _SPLIT turn the cluster forms off as above). */
+typedef struct tfhe_launch {
+    int64_t ciphertexts;
+    int32_t ciphertexts_per_unit;
+    int32_t ctas_per_unit;
+} tfhe_launch;
+int32_t tfhe_keys_launches(const tfhe_keys* keys, int64_t batch, tfhe_launch* launches, int32_t capacity);
 int64_t tfhe_keys_device_bytes(const tfhe_keys* keys);
 
 /* Batched LWE key switch: key_switch_LWE vmapped over ciphertexts

@@ -48,9 +48,10 @@ def _draw(shape, seed, dtype=torch.int32):
     return torch.randint(info.min, info.max, shape, device="cuda", generator=g, dtype=dtype)
 
 
-def _same_as_one_per_cta(keys, batch, seed=0):
+def _same_as_one_per_cta(keys, batch, seed=0, tuning=(0, -1, -1)):
     p = keys.params
     a, b, lut = _draw((batch, p.n), seed), _draw((batch,), seed + 1), _draw((batch, 2, p.N), seed + 2)
+    keys.set_tuning(*tuning)
     got = keys.cuboot_merge(a, b, lut)
     keys.set_tuning(ciphertexts_per_cta=1)
     want = keys.cuboot_merge(a, b, lut)
@@ -130,3 +131,67 @@ def test_a_lost_message_ends_the_cluster(N, n, l_bs, log2_beta, collapse, cluste
     assert t0.elapsed_time(t1) < 10.0
     assert bool((out_a == 77).all()) and bool((out_b == 77).all())
     _same_as_one_per_cta(keys, batch)
+
+
+def _launched(keys, batch):
+    """The number of kernels that a batch's blind rotation launches."""
+    from tfhe_b200.engine import launch_count
+    p = keys.params
+    a, b, lut = _draw((batch, p.n), 1), _draw((batch,), 2), _draw((1, 2, p.N), 3)
+    before = launch_count()
+    keys.cuboot_merge(a, b, lut)
+    return launch_count() - before
+
+
+def _sizes(batch, sms):
+    return batch if batch >= 0 else sms * -batch
+
+
+# (degree, groups x collapse, levels, base, collapse), tuning, {batch (negative: x SMs): launches}
+MMA = (1024, 24, 3, 7, 3)
+FORMS = [
+    (MMA, (0, -1, -1), {1: [(4, 8)], 37: [(4, 8)], 100: [(4, 4)], 200: [(4, 2)], -4: [(4, 1)], 593: [(4, 1), (4, 8)]}),
+    (MMA, (0, -1, 0), {1: [(1, 8)], 30: [(1, 4)], 60: [(1, 2)], 148: [(1, 1)]}),
+    (MMA, (2, -1, -1), {1: [(1, 1)], 200: [(2, 1)]}),
+    ((1024, 24, 3, 9, 3), (0, -1, -1), {1: [(1, 8)], 30: [(1, 4)], 60: [(1, 2)], 148: [(1, 1)], 296: [(2, 1)]}),
+    ((1024, 24, 2, 9, 2), (0, -1, -1), {1: [(1, 8)], 30: [(1, 4)], 60: [(1, 2)], 148: [(1, 1)]}),
+    ((2048, 24, 2, 15, 2), (0, -1, -1), {1: [(1, 8)], 30: [(1, 4)], 60: [(2, 4)], 74: [(1, 2)], 148: [(1, 1)],
+                                         -2: [(2, 1)], -4: [(4, 1)], 593: [(4, 1), (1, 8)]}),
+]
+
+
+@pytest.mark.parametrize("shape,tuning,batches", FORMS)
+def test_launches_say_what_runs(shape, tuning, batches):
+    """Batches for a GPU of 148 SMs; on another only the sums are checked."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    keys = _keys(_params(*shape))
+    for batch, forms in batches.items():
+        batch = _sizes(batch, sms)
+        keys.set_tuning(*tuning)
+        launches = keys.launches(batch)
+        assert sum(x[0] for x in launches) == batch
+        assert len(launches) == _launched(keys, batch)
+        if sms == 148:
+            assert [x[1:] for x in launches] == forms, (batch, launches)
+        _same_as_one_per_cta(keys, batch, tuning=tuning)
+    assert keys.launches(0) == []
+    with pytest.raises(ValueError):
+        keys.launches(-1)
+
+
+def test_launches_say_what_runs64():
+    from tfhe_b200 import client64
+    from tfhe_b200.torus64 import Keys64
+    p = client64.Params64("n24", N=2048, n=24, log2_beta_bs=13, l_bs=2, collapse=3, log2_beta_ks=4, l_ks=5,
+                          sigma_glwe=2.0 ** 17, sigma_lwe=2.0 ** 40)
+    keys = Keys64(client64.keygen(p, 3))
+    for batch, forms in {1: [(1, 8)], 30: [(1, 4)], 60: [(2, 4)], 74: [(1, 2)], 148: [(1, 1)], 296: [(2, 1)],
+                         592: [(4, 1)]}.items():
+        launches = keys.launches(batch)
+        a, b, lut = (_draw(s, 1, torch.int64) for s in ((batch, p.n), (batch,), (1, 2, p.N)))
+        from tfhe_b200.engine import launch_count
+        before = launch_count()
+        keys.cuboot_merge(a, b, lut)
+        assert len(launches) == launch_count() - before and sum(x[0] for x in launches) == batch
+        if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+            assert [x[1:] for x in launches] == forms, (batch, launches)
