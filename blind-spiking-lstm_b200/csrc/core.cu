@@ -702,10 +702,17 @@ static long long mma_cluster_capacity(int L, int M, int C, bool ref) {
     return BM_K * resident_clusters(br_mma_kernel_for(L, M, C, ref), BM_THREADS, br_mma_smem_for(L, M, C), C);
 }
 
+static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStream_t stream,
+                     int* status = nullptr, const tfhe_tuning* tune = nullptr, BrPlan* plan = nullptr);
+
 // Whole rounds of four ciphertexts per SM, then the rest on the widest clusters
-// that hold it in one wave, or a partly filled round (n=630, cycles per group:
-// four per SM 38k, clusters of two 27k for two per SM, of four 18.5k for about
-// one per SM, of eight 11.3k).
+// that hold it in one wave, or a partly filled round.  Between the clusters of
+// eight and of four, and of four and two, the general kernels are the shorter
+// way on the native key (l_bs = 3, eight patterns, cycles per group on 148 SMs:
+// clusters of eight, up to 60 ciphertexts, 11.1k; one per pair, up to 74, 15.5k;
+// clusters of four, up to 132, 18.0k to 19.2k; one per CTA, up to 148, 22.4k;
+// clusters of two, up to 296, 27.3k; four per SM 38.7k).  l_bs = 2 and four
+// patterns stand in the same order.
 static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, const tfhe_tuning* tune,
                       BrPlan* plan = nullptr) {
     const bool ref = args.ct_init != nullptr;
@@ -715,7 +722,10 @@ static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, con
     int C = 0;
     for (int c : {2, 4, 8})
         if (rest > 0 && rest <= mma_cluster_capacity(L, args.M, c, ref)) C = c;
-    const long long head = C ? full : args.B;
+    const bool general = !ref && rest > 0 &&
+                         ((C == 4 && split_applies(N, L, args.G, args.M, rest, false, 0, tune, false)) ||
+                          (C <= 2 && rest <= sm_count()));
+    const long long head = C || general ? full : args.B;
     if (head > 0 && plan) {
         plan->add(head, BM_K, 1);
     } else if (head > 0) {
@@ -735,6 +745,11 @@ static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, con
         count_launch();
         kern<<<(unsigned)std::min<long long>(sets, std::max(1, sm_count())), BM_THREADS, smem, stream>>>(a);
         TFHE_TRY(check_cuda(cudaGetLastError(), "blind rotation launch (matrix instruction)"));
+    }
+    if (general) {
+        BrArgs tail = full ? args_after(args, full, N) : args;
+        tail.bsk_mma = nullptr;
+        return launch_br(tail, N, L, false, 0, stream, nullptr, tune, plan);
     }
     if (!C) return TFHE_OK;
     return launch_cluster(br_mma_kernel_for(L, args.M, C, ref), BM_THREADS, br_mma_smem_for(L, args.M, C), C, BM_K,
@@ -777,7 +792,7 @@ static int launch_warp_four(const BrArgs& args, int N, cudaStream_t stream, cons
 }
 
 static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStream_t stream,
-                     int* status = nullptr, const tfhe_tuning* tune = nullptr, BrPlan* plan = nullptr) {
+                     int* status, const tfhe_tuning* tune, BrPlan* plan) {
     const int logn = ilog2(N);
     const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
     if (mma_takes(args, N, L, tune)) return launch_mma(args, N, L, stream, tune, plan);

@@ -195,3 +195,18 @@ def test_launches_say_what_runs64():
         assert len(launches) == launch_count() - before and sum(x[0] for x in launches) == batch
         if torch.cuda.get_device_properties(0).multi_processor_count == 148:
             assert [x[1:] for x in launches] == forms, (batch, launches)
+
+
+@pytest.mark.parametrize("l_bs,collapse", [(3, 3), (3, 2), (2, 3), (2, 2)])
+def test_n1024_general_kernels_between_the_clusters(l_bs, collapse):
+    """The batches that the general kernels run sooner than the next wider
+    clusters of four ciphertexts, alone and behind whole rounds, and the batches
+    on either side of them."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms != 148:
+        pytest.skip("batches for a GPU of 148 SMs")
+    keys = _keys(_params(1024, 24, l_bs, 7, collapse))
+    for batch, forms in {48: [(4, 8)], 70: [(1, 2)], 74: [(1, 2)], 75: [(4, 4)], 112: [(4, 4)], 148: [(1, 1)],
+                         149: [(4, 2)], 592 + 64: [(4, 1), (1, 2)], 592 + 148: [(4, 1), (1, 1)]}.items():
+        assert [x[1:] for x in keys.launches(batch)] == forms, (batch, keys.launches(batch))
+        _same_as_one_per_cta(keys, batch)
