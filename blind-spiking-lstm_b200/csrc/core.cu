@@ -759,16 +759,21 @@ static int launch_mma(const BrArgs& args, int N, int L, cudaStream_t stream, con
 
 // Ciphertexts of a batch that go to the four-per-CTA kernel in automatic
 // shapes: whole rounds of 4 per SM, and the rest too where a partly filled
-// round is the shortest way (n=742 N=2048, cycles per group and round: four
-// per CTA 44.3k, two 23.4k, one 20.6k; with eight patterns 60.8k, 36.5k and
-// about 30k): above three per SM, with more than four patterns above two.
+// round is the shortest way: above three per SM (eight patterns on the 64-bit
+// torus: two and a half).  Up to there two per CTA and what is left on clusters
+// or one per CTA take as long or less (cycles per
+// group and round, 148 SMs; n=742, four patterns: four per CTA 46.9k, two
+// 24.6k, one 19.8k; eight patterns, 32 bits: 62.5k, 33.5k, 26.8k, and 14.1k to
+// 21.0k for up to 74 on clusters; the 64-bit torus: 64.1k, 37.3k, 27.5k, and
+// 22.4k for 74).
 static long long warp_four_share(int N, int L, int G, int M, long long B, bool reflayout, int kr,
-                                 const tfhe_tuning* tune) {
+                                 const tfhe_tuning* tune, bool t64) {
     const bool requested = (tune && tune->ciphertexts_per_cta > 0) || k_override() > 0;
     if (requested || !persistent_launch(tune) || !warp_form(N, L, G, M, 2, reflayout, kr)) return 0;
     const long long sms = std::max(1, sm_count());
     const long long full = B / (4 * sms) * (4 * sms);
-    return B - full > (M <= 4 ? 3 : 2) * sms ? B : full;
+    const long long rest = B - full;
+    return rest > (t64 && M > 4 ? 5 * sms / 2 : 3 * sms) ? B : full;
 }
 
 static int launch_warp_four(const BrArgs& args, int N, cudaStream_t stream, const tfhe_tuning* tune, BrPlan* plan) {
@@ -816,7 +821,7 @@ static int launch_br(BrArgs args, int N, int L, bool reflayout, int kr, cudaStre
             return launch_br(args_after(args, full, N), N, L, reflayout, kr, stream, status, &rest_tune, plan);
         }
     }
-    if (const long long four = warp_four_share(N, L, args.G, args.M, args.B, reflayout, kr, tune)) {
+    if (const long long four = warp_four_share(N, L, args.G, args.M, args.B, reflayout, kr, tune, args.lwe_a64 != nullptr)) {
         BrArgs head = args;
         head.B = four;
         TFHE_TRY(launch_warp_four(head, N, stream, tune, plan));
@@ -1660,7 +1665,7 @@ int tfhe_pbs_host(const tfhe_keys* keys, const uint32_t* a_host, const uint32_t*
     if (C == 0) {
         const BrShape sh = br_shape(p.N, p.l_bs, keys->M, std::max<long long>(batch, 1 << 20),
                                     keys->tune.ciphertexts_per_cta, true);
-        const long long per_sm = warp_four_share(p.N, p.l_bs, keys->G, keys->M, 1 << 20, false, keys->ring_kr, &keys->tune)
+        const long long per_sm = warp_four_share(p.N, p.l_bs, keys->G, keys->M, 1 << 20, false, keys->ring_kr, &keys->tune, false)
                                      ? 4 : std::max(1, sh.K) * (sh.qtg ? 2 : 1);
         const long long wave = (long long)std::max(1, sm_count()) * per_sm;
         C = std::max<long long>(wave, ((batch + 7) / 8 + wave - 1) / wave * wave);

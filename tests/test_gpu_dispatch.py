@@ -210,3 +210,15 @@ def test_n1024_general_kernels_between_the_clusters(l_bs, collapse):
                          149: [(4, 2)], 592 + 64: [(4, 1), (1, 2)], 592 + 148: [(4, 1), (1, 1)]}.items():
         assert [x[1:] for x in keys.launches(batch)] == forms, (batch, keys.launches(batch))
         _same_as_one_per_cta(keys, batch)
+
+
+@pytest.mark.parametrize("collapse", [2, 3, 4])
+def test_n2048_two_per_cta_up_to_three_per_sm(collapse):
+    """Few ciphertexts above two per SM do not pay for a round of four per CTA."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    keys = _keys(_params(2048, 24, 2, 15, collapse))
+    for batch, first in {2 * sms + 1: (2 * sms, 2, 1), 3 * sms: (2 * sms, 2, 1), 3 * sms + 1: (3 * sms + 1, 4, 1),
+                         6 * sms + 1: (4 * sms, 4, 1)}.items():
+        launches = keys.launches(batch)
+        assert launches[0] == first, (batch, launches)
+        _same_as_one_per_cta(keys, batch)
