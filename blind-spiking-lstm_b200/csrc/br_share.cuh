@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
     // contraction: this lane's point (slot u, block cb of this CTA), output co
     const int co = warp & 1, sl = (warp >> 1) * 32 + lane;
     const int u = rank * NB * 128 + sl;
-    const int pos = key_pos<LOGH>(u);
+    const int pos = key_pos<LOGH, 2>(u);
     const int e = 4 * args.freq[pos] + 1;
     const int cb = sl >> 7, ck2 = pos & 15, cj = ((pos >> 7) & 1) * 4 + ((pos >> 5) & 3);
 

@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) br_warp_kernel(const BrArgs arg
     const int cbase = (wk + cb) * 128 + wh * 64 + 4 * cg;
     // evaluation point zeta^e of the lane's first point; the others' differ by
     // multiples of N / 2 (third digit's bits 3 and 2)
-    const int e0 = 4 * args.freq[key_pos<LOGH>(warp * 128 + lane)] + 1;
+    const int e0 = 4 * args.freq[key_pos<LOGH, L>(warp * 128 + lane)] + 1;
     const int jg = 2 * (cg & 1) + ((cg >> 1) & 1);
 
     const double q = ldexp(1.0, args.log2_q);

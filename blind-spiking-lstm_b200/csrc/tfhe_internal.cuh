@@ -115,14 +115,20 @@ struct Plan {
 __device__ __forceinline__ int swz(int e) { return e ^ (((e >> 3) ^ (e >> 4)) & 7); }
 
 // Storage order of the native Fourier key's H slots: slot u holds position
-// key_pos(u).  At H = 1024 it is the order in which br_warp_kernel's warps
-// contract: slot (warp w, step s, lane) = w 128 + s 32 + lane, so one warp's
-// loads of a step are 1 KB in a row; w, s and lane name the digits of the
-// position (superstages 8.8.16) as that kernel holds them.  The other degrees
-// keep position order.
-template <int LOGH>
+// key_pos(u).  At H = 1024 and l_bs = 2 it is the order in which
+// br_warp_kernel's warps contract: slot (warp w, step s, lane) = w 128 + s 32 +
+// lane, so one warp's loads of a step are 1 KB in a row; w, s and lane name the
+// digits of the position (superstages 8.8.16) as that kernel holds them.  The
+// other degrees and levels keep position order, in which a warp of the cluster
+// kernels reads its digits in rows of 512 bytes, not 64.
+// What the order costs and gives (n=120, four patterns, us): one ciphertext 353
+// in position order, 359 so; 33 ciphertexts 368 and 385; two per CTA (296) 759
+// and 737; four per CTA alike within 0.4%.
+__host__ __device__ constexpr bool key_slots(int logh, int L) { return logh == 10 && L == 2; }
+
+template <int LOGH, int L>
 __host__ __device__ __forceinline__ int key_pos(int u) {
-    if constexpr (LOGH != 10) return u;
+    if constexpr (!key_slots(LOGH, L)) return u;
     const int w = u >> 7, s = (u >> 5) & 3, g = u & 15;
     const int k0 = ((w >> 1) << 1) | ((u >> 4) & 1);                             // first superstage's digit
     const int k1 = (w & 1) | (((g >> 3) & 1) << 1) | (((g >> 2) & 1) << 2);      // second's
@@ -131,8 +137,8 @@ __host__ __device__ __forceinline__ int key_pos(int u) {
 }
 // its inverse
 template <int LOGH>
-__host__ __device__ __forceinline__ int key_slot(int p) {
-    if constexpr (LOGH != 10) return p;
+__host__ __device__ __forceinline__ int key_slot(int p, int L) {
+    if (!key_slots(LOGH, L)) return p;
     const int k0 = p >> 7, k1 = (p >> 4) & 7, k2 = p & 15;
     const int w = ((k0 >> 1) << 1) | (k1 & 1);
     const int s = ((k2 >> 3) & 1) | (((k2 >> 2) & 1) << 1);

@@ -222,3 +222,24 @@ def test_n2048_two_per_cta_up_to_three_per_sm(collapse):
         launches = keys.launches(batch)
         assert launches[0] == first, (batch, launches)
         _same_as_one_per_cta(keys, batch)
+
+
+@pytest.mark.parametrize("l_bs,log2_beta", [(1, 20), (2, 15), (3, 9)])
+def test_fourier_key_is_the_coefficient_key(l_bs, log2_beta):
+    """A key given as spectra lies in the order of the same key given as
+    coefficients, at N = 2048 whatever the levels: the same accumulators."""
+    from tfhe_b200 import client
+    p = _params(2048, 8, l_bs, log2_beta, 2)
+    rng = np.random.default_rng(l_bs)
+    words = lambda shape: rng.integers(0, 2 ** 32, size=shape, dtype=np.uint64).astype(np.uint32)
+    bsk, ka, kb = words((2, 2, p.G * p.M, l_bs, p.N)), words((p.l_ks, p.N, p.n)), words((p.l_ks, p.N))
+    # small key words: both ways round to the same integers
+    bsk = (bsk.view(np.int32) >> 16).view(np.uint32)
+    j = np.arange(p.N)
+    four = np.fft.fft(client._centred(bsk).astype(np.float64) * np.exp(-1j * np.pi * j / p.N))[..., : p.N // 2]
+    ordered = np.ascontiguousarray(four.transpose(1, 0, 3, 2, 4))                   # (out, in, l, G M, N/2)
+    one, two = Keys.create(p, bsk, ka, kb), Keys.create_fourier(p, ordered, ka, kb)
+    for batch in (1, 30, 64, 148, 300, 600):
+        a, b, lut = _draw((batch, p.n), 1), _draw((batch,), 2), _draw((1, 2, p.N), 3)
+        x, y = one.blind_rotate(a, b, lut), two.blind_rotate(a, b, lut)
+        assert torch.equal(x, y), batch
