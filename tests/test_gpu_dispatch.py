@@ -243,3 +243,24 @@ def test_fourier_key_is_the_coefficient_key(l_bs, log2_beta):
         a, b, lut = _draw((batch, p.n), 1), _draw((batch,), 2), _draw((1, 2, p.N), 3)
         x, y = one.blind_rotate(a, b, lut), two.blind_rotate(a, b, lut)
         assert torch.equal(x, y), batch
+
+
+@pytest.mark.parametrize("n,N,l,log2_beta", [(63, 128, 1, 7), (63, 128, 3, 4), (100, 256, 1, 7), (200, 128, 4, 4)])
+def test_short_key_switch_makes_its_digits_in_the_kernel(n, N, l, log2_beta):
+    """One launch where one column tile (or few rows) uses the digits of a short
+    sum, else the digit matrix and the sum; the CUDA cores' words either way."""
+    from tfhe_b200.engine import launch_count
+    p = ParamSet("ks", N=N, n=n, log2_beta_bs=7, l_bs=1, collapse=1, log2_beta_ks=log2_beta, l_ks=l, sigma_glwe=1.0,
+                 sigma_lwe=1.0)
+    keys = _keys(p)
+    for batch in (1, 32, 33, 128, 129, 1000):
+        a, b = _draw((batch, N), batch), _draw((batch,), 7)
+        a.view(-1)[:1] = -2 ** 31
+        before = launch_count()
+        got = keys.keyswitch(a, b)
+        short = N * l < 512 and (4 * (n + 1) <= 256 or batch <= 32)
+        assert launch_count() - before == (1 if short else 2), batch
+        keys.set_tuning(ks_tensor_cores=0)
+        want = keys.keyswitch(a, b)
+        keys.set_tuning()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), batch
