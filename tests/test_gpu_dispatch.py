@@ -264,3 +264,19 @@ def test_short_key_switch_makes_its_digits_in_the_kernel(n, N, l, log2_beta):
         want = keys.keyswitch(a, b)
         keys.set_tuning()
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), batch
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("N", [128, 256, 512, 1024])
+def test_linear_of_many_outputs_is_that_of_few(N, bits):
+    """As many coefficients per thread as the degree has against one: exact sums,
+    so the same words."""
+    from tfhe_b200 import lstm
+    dtype = torch.int32 if bits == 32 else torch.int64
+    J, S = 1201, 2
+    w, bias, x = _draw((J, N), 1), _draw((J,), 2, dtype), _draw((S, 2, N), 3, dtype)
+    w[::3] = 0
+    a, b = lstm.linear_extract(w, bias, x)
+    for j in range(0, J, 100):
+        pa, pb = lstm.linear_extract(w[j: j + 8].contiguous(), bias[j: j + 8].contiguous(), x)
+        assert torch.equal(a[:, j: j + 8], pa) and torch.equal(b[:, j: j + 8], pb), j
