@@ -128,12 +128,13 @@ __global__ void __launch_bounds__(LF_NT) lut_fft_kernel(const int32_t* __restric
     const long long s = blockIdx.y;
     uint32_t* dst = out + (s * Kp + k) * 2 * (long long)N;
 
+    // (over all groups at once: their loads overlap)
     uint32_t most = 0u;
-    for (int g = 0; g < G; ++g)
-        for (int i = tid; i < N; i += nt) {
-            const int v = P[((long long)g * Kp + k) * N + i];
-            most = max(most, v < 0 ? 0u - (uint32_t)v : (uint32_t)v);
-        }
+#pragma unroll 4
+    for (int x = tid; x < G * N; x += nt) {
+        const int v = P[((long long)(x >> LOGN) * Kp + k) * N + (x & (N - 1))];
+        most = max(most, v < 0 ? 0u - (uint32_t)v : (uint32_t)v);
+    }
     if (__syncthreads_or((long long)most * G * N > LF_BOUND)) {
         // direct negacyclic sums (lut_mul_sum_kernel's operations)
         uint32_t* A = reinterpret_cast<uint32_t*>(smem_raw);
@@ -596,7 +597,9 @@ int tfhe_lut_mul_sum(const int32_t* luts, int32_t groups, int32_t per_group, con
                                  : lut_fft_kernel<11>;
         TFHE_TRY(smem_attr_once((const void*)kern, smem));
         count_launch();
-        kern<<<grid, LF_NT, smem, (cudaStream_t)stream>>>(luts, groups, per_group, rlwe, pl->qt, pl->tw, gc, out);
+        // N = 128 has work for 128 threads in the direct sums (1024 products of
+        // large LUTs: 34 us, 62 with 256)
+        kern<<<grid, std::min(LF_NT, N), smem, (cudaStream_t)stream>>>(luts, groups, per_group, rlwe, pl->qt, pl->tw, gc, out);
         return check_cuda(cudaGetLastError(), "lut product launch");
     }
     const size_t smem = 3 * (size_t)N * sizeof(uint32_t);
