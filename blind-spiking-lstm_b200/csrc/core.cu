@@ -189,6 +189,21 @@ static void scratch_trim(int dev) {
     if (dev >= 0 && dev < 64 && g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
 }
 
+const FftPlan* find_plan(int N) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    std::lock_guard<std::mutex> lk(g_plan_mu);
+    auto it = g_plans.find({dev, N});
+    return it != g_plans.end() ? it->second : nullptr;
+}
+
+bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();                                       // the legacy stream during a capture
+    return true;
+}
+
 const FftPlan* get_plan(int N) {
     int dev = 0;
     if (check_cuda(cudaGetDevice(&dev), "cudaGetDevice") != TFHE_OK) return nullptr;

@@ -582,9 +582,9 @@ int tfhe_lut_mul_sum(const int32_t* luts, int32_t groups, int32_t per_group, con
     if (!luts || !rlwe || !out) return fail(TFHE_ERR_INVALID_ARGUMENT, "lut product: null pointer");
     if (S > 65535) return fail(TFHE_ERR_INVALID_ARGUMENT, "lut product: at most 65535 sequences per call");
     const dim3 grid((unsigned)per_group, (unsigned)S);
-    if (N <= 2048) {
-        const FftPlan* pl = get_plan(N);
-        if (!pl) return TFHE_ERR_INTERNAL;
+    // a first call of its degree in a capture cannot build the transform's tables
+    const FftPlan* pl = N > 2048 ? nullptr : capturing((cudaStream_t)stream) ? find_plan(N) : get_plan(N);
+    if (pl) {
         // groups at a time: all that fit in 112 KB, so two blocks share an SM
         const int gc = std::min<int>(groups, std::max<int>(1, (int)((112 * 1024 / (N / 2 * sizeof(double2)) - 2) / 3)));
         const size_t smem = lut_fft_smem(N, gc);

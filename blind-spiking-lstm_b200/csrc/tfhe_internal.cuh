@@ -500,6 +500,11 @@ struct FftPlan {
 
 // returns nullptr (and sets the error) when the table cannot be built
 const FftPlan* get_plan(int N);
+// the same without building it: nullptr when this device has none of that degree
+const FftPlan* find_plan(int N);
+// whether work on this stream is being captured in a graph (or must not be
+// allocated for): no cudaMalloc then
+bool capturing(cudaStream_t stream);
 
 // host helpers used by the launchers
 int plan_tw_count(int logh);

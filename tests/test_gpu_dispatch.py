@@ -280,3 +280,40 @@ def test_linear_of_many_outputs_is_that_of_few(N, bits):
     for j in range(0, J, 100):
         pa, pb = lstm.linear_extract(w[j: j + 8].contiguous(), bias[j: j + 8].contiguous(), x)
         assert torch.equal(a[:, j: j + 8], pa) and torch.equal(b[:, j: j + 8], pb), j
+
+
+FIRST_IN_CAPTURE = """
+import sys, numpy as np, torch
+sys.path[:0] = {paths!r}
+from tfhe_b200 import lstm
+N, G, K, S = {N}, 2, 3, 2
+rng = np.random.default_rng(0)
+lut = torch.from_numpy(rng.integers(-1, 2, size=(G, K, N)).astype(np.int32)).cuda()
+x = torch.from_numpy(rng.integers(-2 ** 31, 2 ** 31, size=(S, G, K, 2, N)).astype(np.int32)).cuda()
+out = torch.zeros((S, K, 2, N), dtype=torch.int32, device="cuda")
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    lstm.lut_mul_sum(lut, x, out=out)
+graph.replay()
+torch.cuda.synchronize()
+first = out.clone()
+assert torch.equal(lstm.lut_mul_sum(lut, x), first) and bool(first.any())
+graph.replay()
+torch.cuda.synchronize()
+assert torch.equal(out, first)
+print("equal")
+"""
+
+
+@pytest.mark.parametrize("N", [256, 2048])
+def test_lut_products_first_called_in_a_capture(N):
+    """Without keys of its degree in the process, the first call may be one being
+    captured: direct sums there, the transform's words after it."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = FIRST_IN_CAPTURE.format(N=N, paths=[os.path.join(root, "blind-spiking-lstm_b200")])
+    run = subprocess.run([sys.executable, "-c", code], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True,
+                         timeout=300)
+    assert run.returncode == 0 and run.stdout.strip().endswith("equal"), run.stdout
