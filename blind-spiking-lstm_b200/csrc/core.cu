@@ -1543,7 +1543,10 @@ int tfhe_keyswitch(const tfhe_keys* keys, const uint32_t* a_in, const uint32_t* 
     TFHE_TRY(check_keys(keys));
     if (batch < 0) return fail(TFHE_ERR_INVALID_ARGUMENT, "negative batch");
     if (batch > 0 && (!a_in || !b_in || !a_out || !b_out)) return fail(TFHE_ERR_INVALID_ARGUMENT, "NULL buffer");
-    return launch_ks(keys, a_in, b_in, a_out, b_out, batch, static_cast<cudaStream_t>(stream));
+    // no memory nodes in a caller's graph (one with them is instantiated once
+    // only): captured, the digits are made in the kernel
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return launch_ks(keys, a_in, b_in, a_out, b_out, batch, st, batch > 0 && !capturing(st));
 }
 
 static BrArgs native_args(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32_t* lwe_b, const uint32_t* lut,

@@ -288,8 +288,6 @@ class PBSGraph:
         self.a = torch.zeros((batch, p.big), **i32)
         self.b = torch.zeros((batch,), **i32)
         self.lut = torch.zeros((lut_count, 2, p.N), **i32)
-        self.ka = torch.empty((batch, p.n), **i32)
-        self.kb = torch.empty((batch,), **i32)
         self.out_a = torch.empty((batch, n_lut, p.N), **i32)
         self.out_b = torch.empty((batch, n_lut), **i32)
         self._step()                      # uncaptured: sets kernel attributes
@@ -299,8 +297,9 @@ class PBSGraph:
             self._step()
 
     def _step(self):
-        self.keys.keyswitch(self.a, self.b, self.ka, self.kb)
-        self.keys.cuboot_merge(self.ka, self.kb, self.lut, self.n_lut, self.out_a, self.out_b)
+        # the bootstrap as one call: a captured key switch on its own makes its
+        # digits in the kernel
+        self.keys.pbs(self.a, self.b, self.lut, self.n_lut, self.out_a, self.out_b)
 
     def __call__(self, a, b, lut=None):
         self.a.copy_(a, non_blocking=True)

@@ -154,7 +154,11 @@ int64_t tfhe_keys_device_bytes(const tfhe_keys* keys);
 
 /* Batched LWE key switch: key_switch_LWE vmapped over ciphertexts
  * (schemas/LWE_jax.py:97-117 as called at nn_tfhe/activation.py:150).
- * a_in (batch, n_big), b_in (batch) -> a_out (batch, n), b_out (batch). */
+ * a_in (batch, n_big), b_in (batch) -> a_out (batch, n), b_out (batch).
+ * The digits (at most 192 MB) are allocated stream-ordered on `stream`; in a
+ * stream capture, and where there is no memory for them, they are made in the
+ * kernel instead (slower, the same words), so a captured key switch adds no
+ * memory nodes to its graph. */
 int tfhe_keyswitch(const tfhe_keys* keys, const uint32_t* a_in, const uint32_t* b_in,
                    uint32_t* a_out, uint32_t* b_out, int64_t batch, void* stream);
 
@@ -185,7 +189,8 @@ int tfhe_cuboot_merge(const tfhe_keys* keys, const uint32_t* lwe_a, const uint32
  * a_in (batch, n_big), b_in (batch), lut (lut_count, 2, N)
  * -> out_a (batch, n_lut, N), out_b (batch, n_lut).
  * The key-switched intermediate and the key switch's digits (at most 192 MB)
- * are allocated stream-ordered on `stream`. */
+ * are allocated stream-ordered on `stream` (memory nodes of a captured graph);
+ * without memory for the digits they are made in the kernel. */
 int tfhe_pbs(const tfhe_keys* keys, const uint32_t* a_in, const uint32_t* b_in,
              const uint32_t* lut, int64_t lut_count, int32_t n_lut,
              uint32_t* out_a, uint32_t* out_b, int64_t batch, void* stream);

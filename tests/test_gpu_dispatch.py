@@ -317,3 +317,27 @@ def test_lut_products_first_called_in_a_capture(N):
     run = subprocess.run([sys.executable, "-c", code], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True,
                          timeout=300)
     assert run.returncode == 0 and run.stdout.strip().endswith("equal"), run.stdout
+
+
+def test_a_captured_key_switch_adds_no_memory_nodes():
+    """A graph with memory nodes is instantiated once only; that of a key switch
+    twice, and both give the uncaptured call's words."""
+    import ctypes
+    keys = _keys(_params(1024, 120, 1, 9, 2))
+    a, b = _draw((200, 1024), 1), _draw((200,), 2)
+    want = keys.keyswitch(a, b)
+    out_a, out_b = torch.empty_like(want[0]), torch.empty_like(want[1])
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        keys.keyswitch(a, b, out_a, out_b)
+    rt = ctypes.CDLL("libcudart.so.12")
+    execs = [ctypes.c_void_p(), ctypes.c_void_p()]
+    for ex in execs:
+        assert rt.cudaGraphInstantiate(ctypes.byref(ex), ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_ulonglong(0)) == 0
+    for ex in execs:
+        out_a.zero_()
+        out_b.zero_()
+        assert rt.cudaGraphLaunch(ex, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(out_a, want[0]) and torch.equal(out_b, want[1])
+        assert rt.cudaGraphExecDestroy(ex) == 0
