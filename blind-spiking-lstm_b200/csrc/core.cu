@@ -1371,8 +1371,9 @@ int tfhe_mul_bootstrap(void* stream, const int64_t* ct_init, int64_t ct_elems, c
     // into their layout (n=630: 165 MB, about 80 us), then the native path's
     // launches, X^r from the index (n=630, 32 ciphertexts: 6.3 -> 1.3 ms with
     // the conversion).  The scratch is stream-ordered; where the caller leaves
-    // no memory for it, the key is read in place as below.
-    if (k_override() <= 0 && persistent_launch(nullptr) &&
+    // no memory for it, and in a capture (a graph with memory nodes can be no
+    // child of another), the key is read in place as below.
+    if (!capturing(st) && k_override() <= 0 && persistent_launch(nullptr) &&
         mma_form((int)degree, (int)l, (int)M, (int)log2_beta, (int)log2_q)) {
         double* key = nullptr;
         if (scratch_alloc((void**)&key, (size_t)G * 4 * l * M * D * sizeof(double2), st) == cudaSuccess) {

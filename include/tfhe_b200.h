@@ -82,6 +82,10 @@ const char* tfhe_last_error(void);
  *   indices      int32 (batch, G, M)
  *   out          int64 (batch, 2, N)
  * degree in {128..4096}, l in {1..4}; other values -> INVALID_ARGUMENT.
+ * At N = 1024, log2_q = 32, base <= 2^8, l 2 or 3 and M 4 or 8 the key is laid
+ * out anew in stream-ordered memory of its size (165 MB at n=630); without
+ * memory for it, and in a stream capture, it is read in place (slower, the
+ * same values).
  * log2_q: 2..64 with the reference's float64 semantics (exact for <= 53).
  */
 int tfhe_mul_bootstrap(void* stream,

@@ -319,10 +319,28 @@ def test_lut_products_first_called_in_a_capture(N):
     assert run.returncode == 0 and run.stdout.strip().endswith("equal"), run.stdout
 
 
+def _instantiated_twice(graph):
+    """Two executables of one captured graph, each as a call that launches it and
+    waits; the second instantiation is refused for a graph with memory nodes."""
+    import ctypes
+    rt = ctypes.CDLL("libcudart.so.12")
+    execs = [ctypes.c_void_p(), ctypes.c_void_p()]
+    for ex in execs:
+        assert rt.cudaGraphInstantiate(ctypes.byref(ex), ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_ulonglong(0)) == 0
+
+    def launch(ex):
+        assert rt.cudaGraphLaunch(ex, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        torch.cuda.synchronize()
+
+    for ex in execs:
+        yield lambda: launch(ex)
+    for ex in execs:
+        assert rt.cudaGraphExecDestroy(ex) == 0
+
+
 def test_a_captured_key_switch_adds_no_memory_nodes():
     """A graph with memory nodes is instantiated once only; that of a key switch
     twice, and both give the uncaptured call's words."""
-    import ctypes
     keys = _keys(_params(1024, 120, 1, 9, 2))
     a, b = _draw((200, 1024), 1), _draw((200,), 2)
     want = keys.keyswitch(a, b)
@@ -330,14 +348,41 @@ def test_a_captured_key_switch_adds_no_memory_nodes():
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph):
         keys.keyswitch(a, b, out_a, out_b)
-    rt = ctypes.CDLL("libcudart.so.12")
-    execs = [ctypes.c_void_p(), ctypes.c_void_p()]
-    for ex in execs:
-        assert rt.cudaGraphInstantiate(ctypes.byref(ex), ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_ulonglong(0)) == 0
-    for ex in execs:
+    for launch in _instantiated_twice(graph):
         out_a.zero_()
         out_b.zero_()
-        assert rt.cudaGraphLaunch(ex, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
-        torch.cuda.synchronize()
+        launch()
         assert torch.equal(out_a, want[0]) and torch.equal(out_b, want[1])
-        assert rt.cudaGraphExecDestroy(ex) == 0
+
+
+def _dropin(l_bs, log2_beta, collapse, n=24):
+    """The drop-in's arguments (BSK, rot) for a uniform key of small words, as the
+    reference holds them, at N = 1024."""
+    N, G = 1024, n // collapse
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    coeff = torch.randint(-2 ** 15, 2 ** 15, (2, 2, G << collapse, l_bs, N), device="cuda", generator=g).to(torch.float64)
+    j = torch.arange(N, device="cuda", dtype=torch.float64)
+    four = torch.fft.fft(coeff * torch.exp(-1j * np.pi * j / N))[..., : N // 2].permute(1, 0, 3, 2, 4).contiguous()
+    angle = (torch.arange(2 * N, device="cuda")[:, None] * (2 * torch.arange(N // 2, device="cuda") + 1)) % (2 * N)
+    return four, torch.exp(-1j * np.pi * angle.to(torch.float64) / N)
+
+
+@pytest.mark.parametrize("l_bs,collapse", [(3, 3), (3, 2), (2, 3), (2, 2)])
+def test_a_captured_dropin_adds_no_memory_nodes(l_bs, collapse):
+    """The drop-in reads its key in place in a capture and lays it out anew
+    elsewhere: the same values, and a graph that is instantiated twice."""
+    from tfhe_b200 import ops
+    four, rot = _dropin(l_bs, 7, collapse)
+    for batch in (1, 5, 150):
+        a, lut = _draw((batch, 24), 1).to(torch.float64), _draw((batch, 2, 1024), 2).to(torch.float64)
+        call = lambda: ops.multiply_seq_monomial(lut, a, four, 32, 7, l_bs, 1024, collapse, rot, 1)
+        want = call()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            out = call()
+        for launch in _instantiated_twice(graph):
+            out.zero_()
+            launch()
+            assert torch.equal(out, want), batch
