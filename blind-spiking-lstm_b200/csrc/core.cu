@@ -148,7 +148,9 @@ int* device_status_word() {
 // up to SCRATCH_KEEP bytes over a synchronisation.  The device's default pool
 // keeps none: each first call after one paid for mapping its memory again
 // (0.5 to 1 ms for a small bootstrap, 2 ms for the drop-in's 165 MB).  The kept
-// memory goes back when a key set is destroyed, and at exit.
+// memory goes back when a key set or packing key is destroyed, by
+// tfhe_trim_working_memory (a caller of the drop-in alone holds no keys), and at
+// exit.
 constexpr uint64_t SCRATCH_KEEP = 256ull << 20;
 static std::mutex g_pool_mu;
 static cudaMemPool_t g_pool[64];
@@ -184,9 +186,10 @@ void scratch_ready() {
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) scratch_pool(dev);
 }
 
-static void scratch_trim(int dev) {
+int scratch_trim(int dev) {
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    if (dev >= 0 && dev < 64 && g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
+    if (dev < 0 || dev >= 64 || !g_pool[dev]) return TFHE_OK;
+    return check_cuda(cudaMemPoolTrimTo(g_pool[dev], 0), "cudaMemPoolTrimTo(working memory)");
 }
 
 const FftPlan* find_plan(int N) {
@@ -1841,6 +1844,15 @@ int32_t tfhe_keys_launches(const tfhe_keys* keys, int64_t batch, tfhe_launch* la
         return -1;
     for (int i = 0; i < std::min<int>(plan.n, std::min<int>(capacity, BrPlan::MAX)); ++i) launches[i] = plan.at[i];
     return plan.n;
+}
+
+int tfhe_trim_working_memory(void) {
+    int rc = TFHE_OK;
+    for (int dev = 0; dev < 64; ++dev) {
+        const int r = scratch_trim(dev);
+        if (rc == TFHE_OK) rc = r;
+    }
+    return rc;
 }
 
 int64_t tfhe_launch_count(void) { return launch_count(); }

@@ -728,6 +728,7 @@ int tfhe_packing_key_destroy(tfhe_packing_key* key) {
     if (!key) return TFHE_OK;
     cudaFree(key->ksp);
     cudaFree(key->limbs);
+    scratch_trim(key->device);
     delete key;
     return TFHE_OK;
 }

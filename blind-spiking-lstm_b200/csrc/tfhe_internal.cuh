@@ -49,6 +49,8 @@ cudaError_t scratch_alloc(void** out, size_t bytes, cudaStream_t stream);
 // makes the pool of the current device (keys and plans call it, so that the
 // first call that needs working memory may be one captured in a graph)
 void scratch_ready();
+// gives back the memory that the pool of a device keeps and no call uses
+int scratch_trim(int dev);
 int check_cuda(cudaError_t e, const char* what);
 
 // ----------------------------------------------------------------------------

@@ -252,6 +252,12 @@ def launch_count() -> int:
     return int(_lib.load().tfhe_launch_count())
 
 
+def trim_working_memory() -> None:
+    """Give the device memory that the library keeps between calls (at most 256
+    MB per device) back to the driver; calls still in flight keep theirs."""
+    _lib.check(_lib.load().tfhe_trim_working_memory())
+
+
 def probe_fp64_peak(iters=4096, reps=5) -> float:
     """Measured FP64 FMA throughput of the current device in TFLOP/s (best
     of ``reps`` launches of 8 independent FMA chains per thread, 8 CTAs of

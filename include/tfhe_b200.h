@@ -250,6 +250,13 @@ int tfhe_device_status(int32_t* status_out, int32_t clear);
  * the number of the library's kernel launches in it. */
 int64_t tfhe_launch_count(void);
 
+/* Calls that need working memory take it stream-ordered from a pool of the
+ * library's own per device, which keeps up to 256 MB between calls (no
+ * counterpart in the reference).  Destroying a key set or packing key gives
+ * back what no call uses; this does so at any time, on every device (the
+ * drop-in's callers hold no keys).  Memory of calls still in flight stays. */
+int tfhe_trim_working_memory(void);
+
 /* Diagnostics (no counterpart in the reference): runs one bounded mbarrier
  * wait that nothing completes, with a limit of limit_cycles clock cycles;
  * *waited_out = 0 when it gave up (the device status then reads

@@ -386,3 +386,20 @@ def test_a_captured_dropin_adds_no_memory_nodes(l_bs, collapse):
             out.zero_()
             launch()
             assert torch.equal(out, want), batch
+
+
+def test_working_memory_goes_back_without_keys():
+    """A caller of the drop-in alone holds no key set: what its call left in the
+    library's pool goes back on request, and the next call takes it anew."""
+    from tfhe_b200 import ops
+    from tfhe_b200.engine import trim_working_memory
+    four, rot = _dropin(3, 7, 3, n=240)
+    scratch = four.numel() * 16
+    a, lut = _draw((2, 240), 1).to(torch.float64), _draw((2, 2, 1024), 2).to(torch.float64)
+    call = lambda: ops.multiply_seq_monomial(lut, a, four, 32, 7, 3, 1024, 3, rot, 1)
+    want = call()
+    torch.cuda.synchronize()
+    kept = torch.cuda.mem_get_info()[0]
+    trim_working_memory()
+    assert torch.cuda.mem_get_info()[0] - kept >= scratch
+    assert torch.equal(call(), want)
