@@ -403,3 +403,61 @@ def test_working_memory_goes_back_without_keys():
     trim_working_memory()
     assert torch.cuda.mem_get_info()[0] - kept >= scratch
     assert torch.equal(call(), want)
+
+
+def test_forms_without_working_memory():
+    """Calls at the limit of the device's memory: the key switch and packing make
+    their digits in the kernel, the drop-in reads its key in place; the same words
+    as with memory."""
+    from tfhe_b200 import client64, lstm, ops, torus64
+    from tfhe_b200.engine import launch_count, trim_working_memory
+    rng = np.random.default_rng(0)
+    words = lambda shape: rng.integers(0, 2 ** 32, size=shape, dtype=np.uint64).astype(np.uint32)
+    keys = _keys(_params(1024, 120, 1, 9, 2))
+    p64 = client64.Params64("ks64", N=1024, n=70, log2_beta_bs=13, l_bs=2, collapse=1, log2_beta_ks=4, l_ks=5,
+                            sigma_glwe=2.0 ** 17, sigma_lwe=2.0 ** 40)
+    keys64 = torus64.Keys64(client64.keygen(p64, 3))
+    pack = lstm.PackingKey(words((1024, 4, 2, 1024)), 7, 4)
+    pack64 = torus64.PackingKey64(rng.integers(0, 2 ** 63, size=(1024, 2, 2, 1024), dtype=np.uint64), 7, 2)
+    four, rot = _dropin(3, 7, 3, n=240)
+    B = 20000
+    a, b = _draw((B, 1024), 1), _draw((B,), 2)
+    a64, b64 = _draw((B, 1024), 3, torch.int64), _draw((B,), 4, torch.int64)
+    idx, lut = torch.randint(0, 2048, (5, 80, 8), dtype=torch.int32, device="cuda"), _draw((5, 2, 1024), 5).to(torch.int64)
+    bsk = four.reshape(2, 2, 3, 80, 8, 512).permute(3, 0, 2, 1, 4, 5).contiguous()
+    import ctypes
+    from tfhe_b200 import _lib
+    out = torch.empty((5, 2, 1024), dtype=torch.int64, device="cuda")
+
+    def dropin():
+        ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+        _lib.check(_lib.load().tfhe_mul_bootstrap(
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ptr(lut), lut.numel(), ptr(bsk),
+            (ctypes.c_int64 * 6)(*bsk.shape), ptr(rot), 2048, ptr(idx), 7, 32, 3, 1024, ptr(out), 5))
+        return out
+
+    outs = [torch.empty((B, 120), dtype=torch.int32, device="cuda"), torch.empty((B,), dtype=torch.int32, device="cuda"),
+            torch.empty((B, 70), dtype=torch.int64, device="cuda"), torch.empty((B,), dtype=torch.int64, device="cuda"),
+            torch.empty((100, 2, 1024), dtype=torch.int32, device="cuda"),
+            torch.empty((100, 2, 1024), dtype=torch.int64, device="cuda")]
+    calls = [lambda: keys.keyswitch(a, b, outs[0], outs[1]), lambda: keys64.keyswitch(a64, b64, outs[2], outs[3], tensor_cores=1),
+             lambda: pack.pack(a.view(100, 200, 1024), b.view(100, 200), out=outs[4]),
+             lambda: pack64.pack(a64.view(100, 200, 1024), b64.view(100, 200), out=outs[5], tensor_cores=1), dropin]
+
+    def run(call):
+        before = launch_count()
+        got = call()
+        torch.cuda.synchronize()
+        got = got if isinstance(got, tuple) else (got,)
+        return [t.cpu() for t in got], launch_count() - before
+
+    want = [run(call) for call in calls]
+    trim_working_memory()
+    hog = Hog(16 << 20)
+    try:
+        got = [run(call) for call in calls]
+    finally:
+        hog.close()
+    for i, ((w, more), (g, launches)) in enumerate(zip(want, got)):
+        assert launches < more, (i, launches, more)          # no digit matrix, no second layout
+        assert all(torch.equal(x, y) for x, y in zip(w, g)), i
