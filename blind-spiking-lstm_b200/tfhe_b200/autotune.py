@@ -3,8 +3,10 @@
 For a key set and a batch size it times the candidate shapes (ciphertexts
 per CTA, L1 prefetch of key words, persistent CTAs) with CUDA events on a
 representative batch, applies the fastest to the keys and records it in a
-JSON cache keyed by GPU name, parameter set and batch bucket, so later
-processes apply it without timing.  Shapes change speed only, never results.
+JSON cache keyed by GPU name, parameter set, batch bucket and what the
+library runs automatically there, so later processes apply it without timing,
+and a library with other forms times anew: a pinned shape keeps the keys from
+forms that its timing did not know.  Shapes change speed only, never results.
 """
 from __future__ import annotations
 
@@ -15,6 +17,7 @@ import tempfile
 import numpy as np
 import torch
 
+from . import _lib
 from .engine import Keys
 
 CACHE_PATH = os.environ.get("TFHE_B200_TUNE_CACHE",
@@ -31,7 +34,9 @@ def bucket(batch: int) -> int:
 
 def _key(keys: Keys, batch: int) -> str:
     name = torch.cuda.get_device_name(torch.cuda.current_device())
-    return f"{name}|{keys.params.name}|{bucket(batch)}"
+    keys.set_tuning()
+    forms = ",".join(f"{k}/{c}" for _, k, c in keys.launches(bucket(batch)))
+    return f"{name}|{keys.params.name}|{bucket(batch)}|{_lib.version()}|{forms}"
 
 
 def load_cache(path: str = CACHE_PATH) -> dict:
