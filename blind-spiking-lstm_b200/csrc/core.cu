@@ -250,7 +250,7 @@ size_t br_table_bytes(int N) {
            (size_t)H * sizeof(uint16_t);
 }
 
-static int sm_count() {
+int sm_count() {
     static int cached[64] = {0};
     int dev = 0;
     cudaGetDevice(&dev);

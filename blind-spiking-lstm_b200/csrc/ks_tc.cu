@@ -884,7 +884,7 @@ static int launch_l3(const KsTcArgs& args, cudaStream_t stream, bool* no_memory)
         *no_memory = true;
         return TFHE_OK;
     }
-    const long long sms = 148, ct = args.npad / KTC_N;
+    const long long sms = std::max(1, sm_count()), ct = args.npad / KTC_N;
     const int all_steps = (int)((K + KT3_K - 1) / KT3_K);
     int rc = TFHE_OK;
     for (long long first = 0; rc == TFHE_OK && first < args.B; first += chunk) {
@@ -1027,7 +1027,7 @@ int build_limbs64(const unsigned long long* key, long long K, int cols, int npad
                   cudaStream_t stream) {
     scratch_ready();
     const long long total = (long long)npad / 8 * K;
-    const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 32);
+    const int blocks = (int)std::min<long long>((total + 255) / 256, std::max(1, sm_count()) * 32LL);
     count_launch();
     limbs64_kernel<<<blocks, 256, 0, stream>>>(key, K, cols, npad, limbs);
     return check_cuda(cudaGetLastError(), "64-bit limb launch");
@@ -1056,7 +1056,7 @@ __global__ void packing_limbs_kernel(const uint32_t* __restrict__ ksp, int n_dim
 int build_packing_limbs(const uint32_t* ksp, int n_dim, int l, int N, int8_t* limbs, cudaStream_t stream) {
     scratch_ready();
     const long long total = 2LL * N * n_dim * l;
-    const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 32);
+    const int blocks = (int)std::min<long long>((total + 255) / 256, std::max(1, sm_count()) * 32LL);
     count_launch();
     packing_limbs_kernel<<<blocks, 256, 0, stream>>>(ksp, n_dim, l, N, limbs);
     return check_cuda(cudaGetLastError(), "packing limb launch");

@@ -139,7 +139,7 @@ int launch_linear(const int32_t* W, const Signed* bias, int J, const Word* ct, l
     const long long tiles = (long long)((J + LIN_JT - 1) / LIN_JT) * S;
     int cpt = 4;
     while (cpt > 1 && LIN_NT * cpt > N) cpt /= 2;
-    while (cpt > 1 && tiles * ((N + LIN_NT * cpt - 1) / (LIN_NT * cpt)) < 296) cpt /= 2;
+    while (cpt > 1 && tiles * ((N + LIN_NT * cpt - 1) / (LIN_NT * cpt)) < 2 * sm_count()) cpt /= 2;
     auto kern = cpt == 4 ? linear_kernel<Word, Signed, 4> : cpt == 2 ? linear_kernel<Word, Signed, 2>
                                                                      : linear_kernel<Word, Signed, 1>;
     const size_t smem = linear_smem<Word>(N, cpt);

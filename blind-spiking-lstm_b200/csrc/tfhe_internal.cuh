@@ -500,6 +500,9 @@ struct FftPlan {
     int tw_count = 0;
 };
 
+// SMs of the current device
+int sm_count();
+
 // returns nullptr (and sets the error) when the table cannot be built
 const FftPlan* get_plan(int N);
 // the same without building it: nullptr when this device has none of that degree
