@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
     uint16_t* rot = reinterpret_cast<uint16_t*>(node + (8 + 64) * BM_NODE);   // [BM_ROT_GROUPS][K][M]
     uint64_t* bars = reinterpret_cast<uint64_t*>(rot + BM_ROT_GROUPS * K * M);   // digits, outputs
     int* bexp = reinterpret_cast<int*>(bars + 2);                    // NC
+    volatile int* gave_up = bexp + 2;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = (int)cluster_rank();
@@ -177,6 +178,7 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         mbar_fence_init();
+        *gave_up = 0;
     }
     cluster_barrier();                                               // tables and barriers ready, every CTA has started
     // bytes that reach this CTA per group
@@ -245,9 +247,11 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
     };
 
     uint32_t phase = 0;                                              // of both barriers, one per group
-    // A wait that runs out ends the loop at the CTA's next barrier, before it
-    // sends anything more; the others' waits for it then run out too, so a
-    // cluster ends within a few limits.  Its outputs are not written.
+    // A wait that runs out ends the loop with its group (the flag is read behind
+    // the group's last barrier and asked for at its end, off the chain); the others'
+    // waits for the next digits then run out too, so a cluster ends within a few
+    // limits.  Outputs that miss anything are not written: in the last group a CTA
+    // whose digits did not come sends no results.
     bool came = true, lost = false;
     for (long long iter = 0; iter < my_sets && !lost; ++iter) {
         const long long ct0 = (cl + iter * ncl) * K;
@@ -444,8 +448,12 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
             }
             // every point of this CTA's outputs is here
             if constexpr (S::ASYNC) {
-                lost = __syncthreads_or(!came);
-                if (lost) break;
+                if (g + 1 < args.G) {
+                    __syncthreads();
+                } else {
+                    lost = __syncthreads_or(!came);
+                    if (lost) break;
+                }
 #pragma unroll
                 for (int i = 0; i < 8 * PPC / BM_THREADS; ++i) {
                     const int o = (tid + i * BM_THREADS) / PPC, e = (tid + i * BM_THREADS) % PPC, p = rank * PPC + e;
@@ -453,7 +461,8 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
                     st_async(peer_smem(out + (size_t)out_poly(0, a) * H + (p ^ ((p >> 3) & 7) ^ a), (uint32_t)dst_rank),
                              gather[o * PPC + (e ^ ((e >> 3) & 7) ^ o)], peer_smem(&bars[1], (uint32_t)dst_rank));
                 }
-                came = bmc_wait(&bars[1], phase, args.wait_limit, args.status);
+                came = came && bmc_wait(&bars[1], phase, args.wait_limit, args.status);
+                if (!came) *gave_up = 1;
             } else {
                 cluster_barrier();
             }
@@ -482,12 +491,8 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
 #pragma unroll
                 for (int j = 0; j < 8; ++j) poly[at(pq, x2, blk * 64 + t8 + 8 * j)] = v[j];
             }
-            if constexpr (S::ASYNC) {
-                lost = __syncthreads_or(!came);
-                if (lost) break;
-            } else {
-                __syncthreads();
-            }
+            __syncthreads();
+            const int ended = S::ASYNC ? *gave_up : 0;
 
             // last superstage, untwist, round, centred reduction (every level's threads)
             if (owner) {
@@ -509,6 +514,8 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
 #pragma unroll
                 for (int n = 0; n < 8; ++n) acc_lo[n] = acc_hi[n] = 0.0;
             }
+            lost = ended;
+            if (lost) break;
         }
         if (lost) break;
         __syncthreads();                                             // dig and out are reused below

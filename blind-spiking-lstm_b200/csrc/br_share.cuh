@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
     uint64_t* bars = reinterpret_cast<uint64_t*>(tw + PL::TW);       // digits, outputs, key words
     uint16_t* rot = reinterpret_cast<uint16_t*>(bars + 3);           // [BS_ROT_GROUPS][K][M]
     int* bexp = reinterpret_cast<int*>(rot + BS_ROT_GROUPS * K * M);
+    volatile int* gave_up = bexp + 2;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = (int)cluster_rank();
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
     if (tid == 0) {
         for (int i = 0; i < 3; ++i) mbar_init(&bars[i], 1);
         mbar_fence_init();
+        *gave_up = 0;
     }
     cluster_barrier();                                               // tables and barriers ready, every CTA has started
     constexpr uint32_t DIGIT_BYTES = NB * K * P * 128 * sizeof(double2), OUT_BYTES = H * sizeof(double2);
@@ -225,7 +227,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
     copy(0);
 
     uint32_t phase = 0;                                              // of all barriers, one per group
-    // a wait that runs out ends the loop at the CTA's next barrier (see
+    // a wait that runs out ends the loop with its group (see
     // br_mma_cluster_kernel)
     bool came = true, lost = false;
     for (int g = 0; g < args.G; ++g, phase ^= 1) {
@@ -359,11 +361,13 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
 #pragma unroll
             for (int i = 0; i < K; ++i) gat[rec_at((cb * K + i) * 2 + co, ck2, cj)] = s[i];
         }
-        lost = __syncthreads_or(!came);
-        if (lost) break;
         if (g + 1 < args.G) {
+            __syncthreads();
             fence_proxy_async_smem();
             copy(g + 1);
+        } else {
+            lost = __syncthreads_or(!came);
+            if (lost) break;
         }
 
         // inverse radix 16 of this CTA's blocks, its points to the polynomials' CTAs
@@ -379,7 +383,8 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
                 st_async(dst + (uint32_t)(out_at(rank * NB + b, 4 * kk + 2 * h2 + h, j) * sizeof(double2)),
                          r[((kk & 1) << 1) | (kk >> 1)], bar);
         }
-        came = bmc_wait(&bars[1], phase, args.wait_limit, args.status);
+        came = came && bmc_wait(&bars[1], phase, args.wait_limit, args.status);
+        if (!came) *gave_up = 1;
 
         // inverse second superstage: butterfly (k0, n)
         if (lvl == 0) {
@@ -393,11 +398,8 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
 #pragma unroll
             for (int k1 = 0; k1 < 8; ++k1) op[out_at((k0 >> 1) * 2 + (k1 & 1), n, (k0 & 1) * 4 + (k1 >> 1))] = v[k1];
         }
-        lost = __syncthreads_or(!came);
-        if (lost) {
-            if (g + 1 < args.G) phase ^= 1;                          // of the key words on their way
-            break;
-        }
+        __syncthreads();
+        const int ended = *gave_up;
 
         // last superstage, untwist, round, centred reduction (both levels' threads)
         if (owner) {
@@ -420,6 +422,11 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
             // written on every path, so nothing is held between here and there
 #pragma unroll
             for (int n2 = 0; n2 < 8; ++n2) acc_lo[n2] = acc_hi[n2] = 0.0;
+        }
+        lost = ended;
+        if (lost) {
+            if (g + 1 < args.G) phase ^= 1;                          // of the key words on their way
+            break;
         }
     }
 
