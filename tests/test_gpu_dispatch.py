@@ -461,3 +461,58 @@ def test_forms_without_working_memory():
     for i, ((w, more), (g, launches)) in enumerate(zip(want, got)):
         assert launches < more, (i, launches, more)          # no digit matrix, no second layout
         assert all(torch.equal(x, y) for x, y in zip(w, g)), i
+
+
+@pytest.mark.parametrize("shape", [(2048, 24, 2, 15, 2), (1024, 24, 3, 7, 3)])
+def test_captured_bootstraps_replay_the_same_words(shape):
+    """Every form of a degree inside a graph: new inputs in the captured buffers,
+    the uncaptured call's words."""
+    keys = _keys(_params(*shape))
+    p = keys.params
+    for batch in (1, 30, 60, 74, 148, 296, 600):
+        a, b, lut = _draw((batch, p.N), 1), _draw((batch,), 2), _draw((batch, 2, p.N), 3)
+        keys.pbs(a, b, lut)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = keys.pbs(a, b, lut)
+        for seed in (4, 5):
+            a.copy_(_draw((batch, p.N), seed))
+            lut.copy_(_draw((batch, 2, p.N), seed + 9))
+            graph.replay()
+            want = keys.pbs(a, b, lut)
+            assert torch.equal(out[0], want[0]) and torch.equal(out[1], want[1]), batch
+        del graph
+
+
+def test_two_streams_at_once():
+    """Bootstraps, key switches, packing and traces whose kernels share the SMs
+    (and their tensor memory) from two streams: each the words it has alone."""
+    from tfhe_b200 import lstm, torus64
+    rng = np.random.default_rng(1)
+    words = lambda shape: rng.integers(0, 2 ** 32, size=shape, dtype=np.uint64).astype(np.uint32)
+    keys = _keys(_params(2048, 24, 2, 15, 2))
+    small = _keys(_params(1024, 24, 3, 7, 3))
+    pack = lstm.PackingKey(words((1024, 4, 2, 1024)), 7, 4)
+    galois = torus64.GaloisKeys64(rng.integers(0, 2 ** 63, size=(11, 5, 2, 2048), dtype=np.uint64), 8, 5)
+    a, b, lut = _draw((700, 2048), 1), _draw((700,), 2), _draw((1, 2, 2048), 3)
+    c, d, lut1 = _draw((40, 1024), 4), _draw((40,), 5), _draw((1, 2, 1024), 6)
+    x, y = _draw((4, 128, 1024), 7), _draw((4, 128), 8)
+    u, v = _draw((40, 2048), 9, torch.int64), _draw((40,), 10, torch.int64)
+    first = lambda s=None: keys.pbs(a, b, lut, stream=s)
+    second = lambda s=None: (*keys.keyswitch(a, b, stream=s), pack.pack(x, y, stream=s),
+                             galois.pack_lwe_to_rlwe(u, v, stream=s), *small.pbs(c, d, lut1, stream=s))
+    want = first(), second()
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(5):
+        with torch.cuda.stream(s1):
+            one = first()
+        with torch.cuda.stream(s2):
+            two = [second() for _ in range(3)]
+        got.append((one, two))
+    torch.cuda.synchronize()
+    for one, two in got:
+        assert all(torch.equal(g, w) for g, w in zip(one, want[0]))
+        for t in two:
+            assert all(torch.equal(g, w) for g, w in zip(t, want[1]))
