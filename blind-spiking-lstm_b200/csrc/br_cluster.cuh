@@ -120,8 +120,8 @@ __global__ void __launch_bounds__(BR_CLUSTER_THREADS, 1) br_cluster_kernel(const
     // this thread's key slot in the pointwise stage (a part's slots are its
     // positions): where its digits lie, and its evaluation point zeta^e
     const int u0 = h * PART + tid / TPS;
-    const int pat = swz(key_pos<LOGH, L>(u0));
-    const int e = 4 * args.freq[key_pos<LOGH, L>(u0)] + 1;
+    const int pat = swz(key_pos<LOGH, L, T64>(u0));
+    const int e = 4 * args.freq[key_pos<LOGH, L, T64>(u0)] + 1;
 
     const bool owner = tid < Q8;
     const int on1 = tid;

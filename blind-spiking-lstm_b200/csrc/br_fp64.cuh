@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(KR > 0 ? KR * (1 << LOGN) / 8 : 512, 1) br_fp6
                 for (int t = tid; t < KG * H; t += nt) {
                     const int kg = t % KG;
                     const int u = t / KG;                          // key slot (the reference layout has position order)
-                    const int p = REFLAYOUT ? u : key_pos<LOGH, L>(u);
+                    const int p = REFLAYOUT ? u : key_pos<LOGH, L, T64>(u);
                     double2 d[KT][P];
     #pragma unroll
                     for (int kt = 0; kt < KT; ++kt)
@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(256) bsk_fft_kernel(const BskConvArgs a) {
             di = ((((size_t)g * parts + p / a.ring_nt) * 2 + out) * a.M + m) * P + bc;
             di = di * a.ring_nt + p % a.ring_nt;
         } else {
-            di = ((((size_t)(g * 2 + out) * (P / 2) + bc / 2) * a.M + m) * H + key_slot<LOGH>(p, a.L)) * 2 + (bc & 1);
+            di = ((((size_t)(g * 2 + out) * (P / 2) + bc / 2) * a.M + m) * H + key_slot<LOGH>(p, a.L, a.src64 != nullptr)) * 2 + (bc & 1);
         }
         // times 1/H: a power of two, so every product and sum of the blind
         // rotation comes out exactly 1/H times the unscaled one, and the

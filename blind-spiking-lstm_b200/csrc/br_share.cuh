@@ -8,8 +8,8 @@
 // quarter of the key and each word serves two ciphertexts.
 //
 // The spectrum's 1024 positions k0 128 + k1 16 + k2 (superstages 8.8.16) are cut
-// into eight blocks w = (k0 / 2, k1 mod 2), which are the key's slot blocks
-// (key_pos: 128 slots each); CTA r owns blocks 2 r and 2 r + 1.  A radix-16
+// into eight blocks w = (k0 / 2, k1 mod 2), 128 positions each (warp_pos); CTA r
+// owns blocks 2 r and 2 r + 1, 256 of the key's slots in a row.  A radix-16
 // butterfly lies inside a block, so:
 //   forward: outer radix-8 pass and second superstage as the other kernels, then
 //     a warp that owns two k0's runs their radix-16 butterflies, two lanes each
@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
     // contraction: this lane's point (slot u, block cb of this CTA), output co
     const int co = warp & 1, sl = (warp >> 1) * 32 + lane;
     const int u = rank * NB * 128 + sl;
-    const int pos = key_pos<LOGH, 2>(u);
+    const int pos = warp_pos(u);
+    const int ku = key_slot<LOGH>(pos, 2, T64);                      // in the slots of the CTA's blocks
     const int e = 4 * args.freq[pos] + 1;
     const int cb = sl >> 7, ck2 = pos & 15, cj = ((pos >> 7) & 1) * 4 + ((pos >> 5) & 3);
 
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
                 if (!kept_back) st_async(dst + (uint32_t)(rec_at(row, 2 * kk + h, j) * sizeof(double2)), r[bm_rev3(kk)], bar);
         }
         // the next two patterns' key words are on their way during the waits
-        const double2* kg = args.bsk + (size_t)g * GROUP + (size_t)co * 2 * M * H * 2 + 2 * (size_t)u;
+        const double2* kg = args.bsk + (size_t)g * GROUP + (size_t)co * 2 * M * H * 2 + 2 * (size_t)ku;
         double2 kw[2][P];
         auto load = [&](int m) {
 #pragma unroll
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) br_share_kernel(const BrArgs ar
             for (int m = 0; m < MS; ++m) {
                 double2 k[P];
 #pragma unroll
-                for (int x = 0; x < P; ++x) k[x] = stage[(m * 4 + co * 2 + (x >> 1)) * NB * 256 + 2 * sl + (x & 1)];
+                for (int x = 0; x < P; ++x) k[x] = stage[(m * 4 + co * 2 + (x >> 1)) * NB * 256 + 2 * (ku & (NB * 128 - 1)) + (x & 1)];
                 one(m, k);
             }
 #pragma unroll 1

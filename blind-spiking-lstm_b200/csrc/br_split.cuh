@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(BR_SPLIT_THREADS, 1) br_split_kernel(const BrA
     int at[SL], ev[SL];
 #pragma unroll
     for (int sl = 0; sl < SL; ++sl) {
-        const int p = key_pos<LOGH, L>((tid + sl * BR_SPLIT_THREADS) % H);
+        const int p = key_pos<LOGH, L, T64>((tid + sl * BR_SPLIT_THREADS) % H);
         at[sl] = swz(p);
         ev[sl] = 4 * args.freq[p] + 1;
     }

@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(BR_TM_THREADS, 1) br_tm_kernel(const BrArgs ar
             {
                 const size_t gbase = (size_t)g * 2 * P * M * H;
                 for (int u = tid; u < H; u += nt) {
-                    const int p = key_pos<LOGH, L>(u);
+                    const int p = key_pos<LOGH, L, T64>(u);
                     double2 d[K][P];
 #pragma unroll
                     for (int kt = 0; kt < K; ++kt)

@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) br_warp_kernel(const BrArgs arg
     const int cbase = (wk + cb) * 128 + wh * 64 + 4 * cg;
     // evaluation point zeta^e of the lane's first point; the others' differ by
     // multiples of N / 2 (third digit's bits 3 and 2)
-    const int e0 = 4 * args.freq[key_pos<LOGH, L>(warp * 128 + lane)] + 1;
+    const int e0 = 4 * args.freq[warp_pos(warp * 128 + lane)] + 1;
     const int jg = 2 * (cg & 1) + ((cg >> 1) & 1);
 
     const double q = ldexp(1.0, args.log2_q);
@@ -473,7 +473,11 @@ __global__ void __launch_bounds__(BW_THREADS, 1) br_warp_kernel(const BrArgs arg
             // contraction: out[a] = sum_m X^{r_m} sum_bc BSK[g, a, bc, m] DEC[bc],
             // the key words of two steps (point, pattern) in flight
             {
-                const double2* kb = args.bsk + (size_t)g * 2 * P * M * H + 2 * (warp * 128 + lane);
+                const double2* kb = args.bsk + (size_t)g * 2 * P * M * H + 2 * key_slot<LOGH>(warp_pos(warp * 128 + lane), L, T64);
+                // key words of point s: of position bits 3 and 2, in rows slot bits 4 and 3
+                auto point = [](int s) {
+                    return key_order(LOGH, L, T64) == KEY_STEPS ? 64 * s : 32 * (s & 1) + 16 * (s >> 1);
+                };
                 const uint16_t* rg = rot + g * M * K;
                 const size_t row = (size_t)M * H * 2;
                 double2 kx[2][P], ky[2][P], w[K];
@@ -547,7 +551,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) br_warp_kernel(const BrArgs arg
 #pragma unroll 1
                     for (int m = 0; m < M; m += 2) {
                         const bool last = m + 2 >= M;
-                        const double2* nx = !last ? kb + (size_t)(m + 2) * H * 2 + 64 * s : kb + 64 * (s + 1);
+                        const double2* nx = !last ? kb + (size_t)(m + 2) * H * 2 + point(s) : kb + point(s + 1);
                         const bool more = !last || s < 3;
                         if (m > 0) step(kx, m + 1, e);
                         if (more) load(kx, nx);

@@ -1449,7 +1449,7 @@ int tfhe_keys_create_fourier(const tfhe_params* params, const double* bsk_ordere
                                 di = ((((size_t)g * (H / rnt) + pp / rnt) * 2 + a) * M + m) * P + bc;
                                 di = di * rnt + pp % rnt;
                             } else {
-                                const int u = H == 1024 ? key_slot<10>(pp, L) : pp;
+                                const int u = H == 1024 ? key_slot<10>(pp, L, false) : pp;
                                 di = (((((size_t)g * 2 + a) * (P / 2) + bc / 2) * M + m) * H + u) * 2 + (bc & 1);
                             }
                             // times 1/H, as bsk_fft_kernel stores the native key

@@ -116,31 +116,48 @@ struct Plan {
 // stage take the minimum of 4 wavefronts per 32 16-byte requests.
 __device__ __forceinline__ int swz(int e) { return e ^ (((e >> 3) ^ (e >> 4)) & 7); }
 
-// Storage order of the native Fourier key's H slots: slot u holds position
-// key_pos(u).  At H = 1024 and l_bs = 2 it is the order in which
-// br_warp_kernel's warps contract: slot (warp w, step s, lane) = w 128 + s 32 +
-// lane, so one warp's loads of a step are 1 KB in a row; w, s and lane name the
-// digits of the position (superstages 8.8.16) as that kernel holds them.  The
-// other degrees and levels keep position order, in which a warp of the cluster
-// kernels reads its digits in rows of 512 bytes, not 64.
-// What the order costs and gives (n=120, four patterns, us): one ciphertext 353
-// in position order, 359 so; 33 ciphertexts 368 and 385; two per CTA (296) 759
-// and 737; four per CTA alike within 0.4%.
-__host__ __device__ constexpr bool key_slots(int logh, int L) { return logh == 10 && L == 2; }
-
-template <int LOGH, int L>
-__host__ __device__ __forceinline__ int key_pos(int u) {
-    if constexpr (!key_slots(LOGH, L)) return u;
+// the position k0 128 + k1 16 + k2 (digits of superstages 8.8.16, H = 1024) that
+// warp w, step s and lane of br_warp_kernel contract, of u = w 128 + s 32 + lane: the
+// lanes differ in k2's bits 0 and 1, k1's 1 and 2 and k0's 0, the steps in k2's 3 and 2
+__host__ __device__ __forceinline__ int warp_pos(int u) {
     const int w = u >> 7, s = (u >> 5) & 3, g = u & 15;
-    const int k0 = ((w >> 1) << 1) | ((u >> 4) & 1);                             // first superstage's digit
-    const int k1 = (w & 1) | (((g >> 3) & 1) << 1) | (((g >> 2) & 1) << 2);      // second's
-    const int k2 = ((s & 1) << 3) | ((s >> 1) << 2) | ((g & 1) << 1) | ((g >> 1) & 1);   // third's
+    const int k0 = ((w >> 1) << 1) | ((u >> 4) & 1);
+    const int k1 = (w & 1) | (((g >> 3) & 1) << 1) | (((g >> 2) & 1) << 2);
+    const int k2 = ((s & 1) << 3) | ((s >> 1) << 2) | ((g & 1) << 1) | ((g >> 1) & 1);
     return k0 * 128 + k1 * 16 + k2;
+}
+
+// Storage order of the native Fourier key's H slots: slot u holds position
+// key_pos(u).  Degrees and levels that br_warp_kernel does not take keep position
+// order.  At H = 1024 and l_bs = 2:
+//   32-bit torus, rows: a slot's bits, lowest first, are k2's 0 and 1, k1's 2, k2's 2
+//     and 3, k1's 1 and 0, k0.  br_warp_kernel reads its key words in rows of 256
+//     bytes; the cluster kernels, threads in order of slots, theirs in rows of 1 KB
+//     and the digits, their own and other CTAs', in two rows of 256.
+//   64-bit torus, steps: warp_pos.  br_warp_kernel's rows are 1 KB, a cluster
+//     kernel's warp reads its digits in pieces of 64 bytes.
+// n=120, four patterns, 32 bits, us, in position order / rows / steps: one
+// ciphertext 349 / 356 / 359, 33 368 / 370 / 386, 64 418 / 417 / 425, 74 490 / 489 /
+// 500, two per CTA (296) 759 / 749 / 738, four per CTA (5920) 13905 / 13844 / 13870.
+// Eight patterns, 64 bits, n=24: 33 67 / 67 / 70, four per CTA (4736) 2059 / 2057 /
+// 2048; a layer's timestep of 16 sequences 27.27 / 27.29 / 27.01 ms, hence its steps.
+enum { KEY_POSITIONS, KEY_ROWS, KEY_STEPS };
+__host__ __device__ constexpr int key_order(int logh, int L, bool t64) {
+    return logh != 10 || L != 2 ? KEY_POSITIONS : t64 ? KEY_STEPS : KEY_ROWS;
+}
+
+template <int LOGH, int L, bool T64>
+__host__ __device__ __forceinline__ int key_pos(int u) {
+    if constexpr (key_order(LOGH, L, T64) == KEY_POSITIONS) return u;
+    if constexpr (key_order(LOGH, L, T64) == KEY_STEPS) return warp_pos(u);
+    return (u & 0x383) | ((u & 4) << 4) | ((u & 8) >> 1) | ((u & 16) >> 1) | (u & 32) | ((u & 64) >> 2);
 }
 // its inverse
 template <int LOGH>
-__host__ __device__ __forceinline__ int key_slot(int p, int L) {
-    if (!key_slots(LOGH, L)) return p;
+__host__ __device__ __forceinline__ int key_slot(int p, int L, bool t64) {
+    if (key_order(LOGH, L, t64) == KEY_POSITIONS) return p;
+    if (key_order(LOGH, L, t64) == KEY_ROWS)
+        return (p & 0x383) | ((p & 64) >> 4) | ((p & 4) << 1) | ((p & 8) << 1) | (p & 32) | ((p & 16) << 2);
     const int k0 = p >> 7, k1 = (p >> 4) & 7, k2 = p & 15;
     const int w = ((k0 >> 1) << 1) | (k1 & 1);
     const int s = ((k2 >> 3) & 1) | (((k2 >> 2) & 1) << 1);
