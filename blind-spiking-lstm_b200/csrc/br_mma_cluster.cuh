@@ -149,7 +149,6 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
     uint16_t* rot = reinterpret_cast<uint16_t*>(node + (8 + 64) * BM_NODE);   // [BM_ROT_GROUPS][K][M]
     uint64_t* bars = reinterpret_cast<uint64_t*>(rot + BM_ROT_GROUPS * K * M);   // digits, outputs
     int* bexp = reinterpret_cast<int*>(bars + 2);                    // NC
-    volatile int* gave_up = bexp + 2;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = (int)cluster_rank();
@@ -178,7 +177,6 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         mbar_fence_init();
-        *gave_up = 0;
     }
     cluster_barrier();                                               // tables and barriers ready, every CTA has started
     // bytes that reach this CTA per group
@@ -247,11 +245,15 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
     };
 
     uint32_t phase = 0;                                              // of both barriers, one per group
-    // A wait that runs out ends the loop with its group (the flag is read behind
-    // the group's last barrier and asked for at its end, off the chain); the others'
-    // waits for the next digits then run out too, so a cluster ends within a few
-    // limits.  Outputs that miss anything are not written: in the last group a CTA
-    // whose digits did not come sends no results.
+    // A wait that runs out ends the CTA's loop with its group, by a vote at one of
+    // the group's barriers: the others' waits for the next digits run out too, so a
+    // cluster ends within a few limits.  A CTA that leaves writes no outputs; those
+    // of a call that records a timeout are undefined all the same.  The vote is at
+    // the barrier behind the results' wait for C = 8 and at the one behind the
+    // contraction for C = 4, each where it costs nothing (n=630, us, no vote / behind
+    // the results / behind the contraction: 32 ciphertexts 1142 / 1092 / 1156, 100
+    // ciphertexts 1889 / 1940 / 1890).
+    constexpr bool VOTE_LATE = C == 8;
     bool came = true, lost = false;
     for (long long iter = 0; iter < my_sets && !lost; ++iter) {
         const long long ct0 = (cl + iter * ncl) * K;
@@ -448,12 +450,8 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
             }
             // every point of this CTA's outputs is here
             if constexpr (S::ASYNC) {
-                if (g + 1 < args.G) {
-                    __syncthreads();
-                } else {
-                    lost = __syncthreads_or(!came);
-                    if (lost) break;
-                }
+                if constexpr (VOTE_LATE) __syncthreads();
+                else lost = __syncthreads_or(!came);
 #pragma unroll
                 for (int i = 0; i < 8 * PPC / BM_THREADS; ++i) {
                     const int o = (tid + i * BM_THREADS) / PPC, e = (tid + i * BM_THREADS) % PPC, p = rank * PPC + e;
@@ -461,8 +459,7 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
                     st_async(peer_smem(out + (size_t)out_poly(0, a) * H + (p ^ ((p >> 3) & 7) ^ a), (uint32_t)dst_rank),
                              gather[o * PPC + (e ^ ((e >> 3) & 7) ^ o)], peer_smem(&bars[1], (uint32_t)dst_rank));
                 }
-                came = came && bmc_wait(&bars[1], phase, args.wait_limit, args.status);
-                if (!came) *gave_up = 1;
+                came &= bmc_wait(&bars[1], phase, args.wait_limit, args.status);
             } else {
                 cluster_barrier();
             }
@@ -491,8 +488,8 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
 #pragma unroll
                 for (int j = 0; j < 8; ++j) poly[at(pq, x2, blk * 64 + t8 + 8 * j)] = v[j];
             }
-            __syncthreads();
-            const int ended = S::ASYNC ? *gave_up : 0;
+            if constexpr (VOTE_LATE) lost = __syncthreads_or(!came);
+            else __syncthreads();
 
             // last superstage, untwist, round, centred reduction (every level's threads)
             if (owner) {
@@ -514,11 +511,15 @@ __global__ void __launch_bounds__(BM_THREADS, 1) br_mma_cluster_kernel(const BrA
 #pragma unroll
                 for (int n = 0; n < 8; ++n) acc_lo[n] = acc_hi[n] = 0.0;
             }
-            lost = ended;
-            if (lost) break;
+            if (S::ASYNC && lost) break;
         }
         if (lost) break;
-        __syncthreads();                                             // dig and out are reused below
+        if constexpr (S::ASYNC && !VOTE_LATE) {
+            lost = __syncthreads_or(!came);
+            if (lost) break;
+        } else {
+            __syncthreads();                                         // dig and out are reused below
+        }
 
         if constexpr (REF) {
             if (owner && (!S::LP || olv == 0) && ct0 + ct_in < args.B) {
