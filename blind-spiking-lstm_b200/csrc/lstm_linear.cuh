@@ -76,10 +76,8 @@ __global__ void __launch_bounds__(LIN_NT) linear_kernel(const int32_t* __restric
 #pragma unroll
         for (int r = 0; r < CPT; ++r) acc[jt][r] = 0;
     const Word* e0 = E + (N - 1) + tid;
-    // (warps past the last coefficient, at N < 256, have nothing to add)
-    const int terms = c0 + tid < N ? n : 0;
 #pragma unroll 4
-    for (int i = 0; i < terms; ++i) {
+    for (int i = 0; i < n; ++i) {
         const int4 w = lw[i];
         const Word* e = e0 - lm[i];
 #pragma unroll
@@ -131,7 +129,7 @@ __global__ void __launch_bounds__(LIN_NT) linear_kernel(const int32_t* __restric
 }
 
 // coefficients per thread: as many as leave about two blocks per SM and do not
-// reach past N (N = 128, 1000 outputs of 40 ciphertexts, dense, 64 bits: 267 us, 1622
+// reach past N (N = 128, 1000 outputs of 40 ciphertexts, dense, 64 bits: 450 us, 1622
 // with four)
 template <class Word, class Signed>
 int launch_linear(const int32_t* W, const Signed* bias, int J, const Word* ct, long long S, int N, Word* out_a,
