@@ -34,11 +34,13 @@
 // of the CTA lies between two waits for the same mbarrier, and the second phase
 // needs this CTA's own stores, so no thread misses a phase.
 //
-// n=630 N=1024 with the key switch, ms: batch 1 1.14 (one ciphertext on eight
-// CTAs, br_cluster_kernel, 1.58), 37 1.17 (1.60), 64 1.88 (cluster pair 1.91),
-// 128 1.95 (one CTA each 2.40), 256 2.86 (two per CTA 4.20).  A group at C = 8
-// takes 11.3k cycles: about 3.5k the contraction (1.5k of it matrix issue),
-// the rest the chain of passes and exchanges.
+// n=630 N=1024 with the key switch, ms: batch 1 1.11 (one ciphertext on eight
+// CTAs, br_cluster_kernel, 1.58), 32 1.12 (on four CTAs 1.61), 60 1.15 (cluster
+// pair 1.93), 128 1.97 (one CTA each 2.50), 256 2.89 (two per CTA 4.20); the
+// launcher leaves 61 to 74 to the pair (1.83) and 133 to 148 to one CTA each (2.40).
+// A group at C = 8 takes 10.3k cycles: about 3.5k the contraction (1.5k of it
+// matrix issue), the rest the chain of passes and exchanges (FP64 pipe 19%, FP64
+// matrix pipe 15%).
 #pragma once
 
 #include "br_mma.cuh"

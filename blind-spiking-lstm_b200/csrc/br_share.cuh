@@ -29,11 +29,10 @@
 // two patterns of the next group come by bulk copies while the inverse and the
 // next forward transform run.
 //
-// n=742 with the key switch, ms: 37 ciphertexts 3.15 -> 2.53, 64 3.15 -> 2.59
-// (cluster pair).  About 13k
-// cycles a group, a quarter of them the contraction; the rest is the chain of
-// passes (the last and first superstages 3.4k on eight warps, the middle ones
-// 2.2k) and the two exchanges.  Four ciphertexts per cluster of eight took 2.50 ms, but
+// n=742 with the key switch, ms: 37 ciphertexts 2.43, 64 2.53 (cluster pair
+// 3.08).  About 13k cycles a group, a quarter of them the contraction; the rest
+// is the chain of passes (the last and first superstages 3.4k on eight warps, the
+// middle ones 2.2k) and the two exchanges (FP64 pipe 30%).  Four ciphertexts per cluster of eight took 2.50 ms, but
 // only 14 such clusters are resident; four per cluster of four 4.47 ms.
 //
 // No buffer is written early: a CTA sends digits of group g + 1 only after all its

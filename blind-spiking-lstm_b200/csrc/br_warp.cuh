@@ -31,9 +31,10 @@
 // What bounds it: FP64 issue.  A DFMA takes 2 cycles per warp and scheduler,
 // 2.4 to 2.9 with three distinct register operands, which puts the floor of
 // two ciphertexts' group (n=742: four patterns) at about 16k cycles; measured
-// 22.2k, br_fp64_kernel with 16 warps and two ciphertexts per key word 25.9k
-// (16384 ciphertexts 275 -> 233 ms); with eight patterns on the 64-bit torus
-// 30.4k against 36.5k.  The FP64 pipe is 59% busy (50% before).  Why four
+// 22.9k, br_fp64_kernel with 16 warps and two ciphertexts per key word 25.9k
+// (16384 ciphertexts 275 -> 240 ms); with eight patterns on the 64-bit torus
+// 30.4k against 36.5k.  The FP64 pipe is 58% busy (50% before), the shared-memory
+// pipe 57%.  Why four
 // ciphertexts per key word: with all SMs in step a key word takes about 1100
 // cycles from L2, so eight warps with the key words of two steps in flight
 // draw 50 bytes per cycle; two ciphertexts per word would need twice that.

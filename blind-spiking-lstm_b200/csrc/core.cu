@@ -700,8 +700,11 @@ static bool persistent_launch(const tfhe_tuning* tune) {
 // The matrix-instruction kernels (br_mma.cuh, br_mma_cluster.cuh) take N = 1024
 // on the 32-bit torus, l_bs 2 or 3, four or eight patterns, where the rounded
 // float64 products are the exact integers whatever the order of their sums: at
-// log2 beta = 7 (l_bs = 3, eight patterns) a product is at most 0.03 off its
-// integer, and the error grows with beta.
+// log2 beta = 7 (l_bs = 3, eight patterns) a product of a chain is at most 0.03 off
+// its integer, and the error doubles with beta (40 uniform groups in float64:
+// 0.016 at 7, 0.031 at 8, of the 0.5 that there is).  Measured, not bounded: digits
+// all at their largest against a key aligned to them would leave float64's 53 bits,
+// where every order of the sums rounds differently.
 static bool mma_form(int N, int L, int M, int log2_beta, int log2_q) {
     return N == BM_N && log2_q == 32 && log2_beta <= 8 && (L == 2 || L == 3) && (M == 4 || M == 8) &&
            br_mma_smem_for(L, M, 1) <= (size_t)max_smem_optin();
@@ -1022,7 +1025,7 @@ static int launch_ks_key(const KsKey& key, int n_big, int n, int l, int log2_bet
     // Few ciphertexts give few tiles, each a serial sum over n_big l key rows:
     // the input coefficients are then split over blockIdx.z, up to about two
     // blocks per SM and at least four steps each, the parts added by atomics
-    // (32 ciphertexts, 1024 -> 630, 5 levels: 828 -> 60 us)
+    // (32 ciphertexts, 1024 -> 630, 5 levels: 828 -> 41 us)
     const long long tiles = (long long)((n + 1 + KS_TO - 1) / KS_TO) * ((B + KS_TB - 1) / KS_TB);
     const long long want = std::max<long long>(1, 2 * std::max(1, sm_count()) / tiles);
     const int steps = (n_big + KS_KC - 1) / KS_KC;

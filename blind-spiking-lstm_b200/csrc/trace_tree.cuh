@@ -20,8 +20,8 @@
 //   * the transform's last level and the inverse's first run in the product's
 //     registers, the inverse's outer twiddles and the untwist are one product;
 //   * the words wait in tensor memory while the spectra need the registers.
-// Bound by shared memory and the key loads (LSU data path 71% busy, FP64 41%,
-// issue 38%).  l = 5: 296 LWEs 413 -> 284 us, 512 778 -> 485, 2048 2739 -> 1701,
+// Bound by shared memory and the key loads (1184 LWEs: LSU data path 78% busy,
+// FP64 45%, issue 41%).  l = 5: 296 LWEs 413 -> 284 us, 512 778 -> 485, 2048 2739 -> 1701,
 // one LWE 216 -> 161, against the general kernel.  Two LWEs per CTA with shared
 // key words took 549 us at 512: one CTA's phases leave the SM idle.
 #pragma once
