@@ -151,11 +151,11 @@ def _sizes(batch, sms):
 MMA = (1024, 24, 3, 7, 3)
 FORMS = [
     (MMA, (0, -1, -1), {1: [(4, 8)], 37: [(4, 8)], 100: [(4, 4)], 200: [(4, 2)], -4: [(4, 1)], 593: [(4, 1), (4, 8)]}),
-    (MMA, (0, -1, 0), {1: [(1, 8)], 30: [(1, 4)], 60: [(1, 2)], 148: [(1, 1)]}),
+    (MMA, (0, -1, 0), {1: [(1, 8)], 24: [(1, 4)], 60: [(1, 2)], 148: [(1, 1)]}),
     (MMA, (2, -1, -1), {1: [(1, 1)], 200: [(2, 1)]}),
-    ((1024, 24, 3, 9, 3), (0, -1, -1), {1: [(1, 8)], 30: [(1, 4)], 60: [(1, 2)], 148: [(1, 1)], 296: [(2, 1)]}),
-    ((1024, 24, 2, 9, 2), (0, -1, -1), {1: [(1, 8)], 30: [(1, 4)], 60: [(1, 2)], 148: [(1, 1)]}),
-    ((2048, 24, 2, 15, 2), (0, -1, -1), {1: [(1, 8)], 30: [(1, 4)], 60: [(2, 4)], 74: [(1, 2)], 148: [(1, 1)],
+    ((1024, 24, 3, 9, 3), (0, -1, -1), {1: [(1, 8)], 24: [(1, 4)], 60: [(1, 2)], 148: [(1, 1)], 296: [(2, 1)]}),
+    ((1024, 24, 2, 9, 2), (0, -1, -1), {1: [(1, 8)], 24: [(1, 4)], 60: [(1, 2)], 148: [(1, 1)]}),
+    ((2048, 24, 2, 15, 2), (0, -1, -1), {1: [(1, 8)], 24: [(1, 4)], 56: [(2, 4)], 74: [(1, 2)], 148: [(1, 1)],
                                          -2: [(2, 1)], -4: [(4, 1)], 593: [(4, 1), (1, 8)]}),
 ]
 
@@ -185,7 +185,7 @@ def test_launches_say_what_runs64():
     p = client64.Params64("n24", N=2048, n=24, log2_beta_bs=13, l_bs=2, collapse=3, log2_beta_ks=4, l_ks=5,
                           sigma_glwe=2.0 ** 17, sigma_lwe=2.0 ** 40)
     keys = Keys64(client64.keygen(p, 3))
-    for batch, forms in {1: [(1, 8)], 30: [(1, 4)], 60: [(2, 4)], 74: [(1, 2)], 148: [(1, 1)], 296: [(2, 1)],
+    for batch, forms in {1: [(1, 8)], 24: [(1, 4)], 56: [(2, 4)], 74: [(1, 2)], 148: [(1, 1)], 296: [(2, 1)],
                          592: [(4, 1)]}.items():
         launches = keys.launches(batch)
         a, b, lut = (_draw(s, 1, torch.int64) for s in ((batch, p.n), (batch,), (1, 2, p.N)))
@@ -206,8 +206,8 @@ def test_n1024_general_kernels_between_the_clusters(l_bs, collapse):
     if sms != 148:
         pytest.skip("batches for a GPU of 148 SMs")
     keys = _keys(_params(1024, 24, l_bs, 7, collapse))
-    for batch, forms in {48: [(4, 8)], 70: [(1, 2)], 74: [(1, 2)], 75: [(4, 4)], 112: [(4, 4)], 148: [(1, 1)],
-                         149: [(4, 2)], 592 + 64: [(4, 1), (1, 2)], 592 + 148: [(4, 1), (1, 1)]}.items():
+    for batch, forms in {40: [(4, 8)], 74: [(1, 2)], 75: [(4, 4)], 100: [(4, 4)], 148: [(1, 1)],
+                         149: [(4, 2)], 592 + 74: [(4, 1), (1, 2)], 592 + 148: [(4, 1), (1, 1)]}.items():
         assert [x[1:] for x in keys.launches(batch)] == forms, (batch, keys.launches(batch))
         _same_as_one_per_cta(keys, batch)
 
